@@ -3,8 +3,10 @@
 ``python -m flashoptim_b200.build`` compiles every ``csrc/*.cu`` with nvcc for
 ``sm_100a`` and links one shared library next to the package.  The library has
 no PyTorch dependency: Python passes raw device pointers and the current CUDA
-stream through :mod:`ctypes` (see :mod:`flashoptim_b200.ops.native`).  A stamp
-file holding a hash of sources and flags makes repeated calls free.
+stream through :mod:`ctypes` (see :mod:`flashoptim_b200.ops.native`).  The host
+walk over a parameter group, ``csrc/fo_host.cpp``, is a CPython extension of its
+own, built against the installed PyTorch (:mod:`flashoptim_b200.ops.host`).
+Stamp files holding a hash of sources and flags make repeated calls free.
 """
 
 from __future__ import annotations
@@ -24,6 +26,10 @@ SRC_DIR = PKG_DIR / "csrc"
 LIB_DIR = PKG_DIR / "_lib"
 LIB_PATH = LIB_DIR / "libflashoptim_b200.so"
 STAMP_PATH = LIB_DIR / "build.stamp"
+HOST_SOURCE = SRC_DIR / "fo_host.cpp"
+HOST_PATH = LIB_DIR / "_fo_host.so"
+HOST_STAMP_PATH = LIB_DIR / "host.stamp"
+HOST_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-shared", "-Wno-unknown-pragmas"]
 
 NVCC_FLAGS = [
     "-gencode",
@@ -142,12 +148,74 @@ def _build_locked(nvcc: str, out: Path, default_target: bool, verbose: bool, ext
         if os.path.exists(tmp):
             os.unlink(tmp)
     if default_target:
-        stamp_tmp = STAMP_PATH.with_suffix(".stamp.tmp")
-        stamp_tmp.write_text(source_hash(extra_flags))
-        os.replace(stamp_tmp, STAMP_PATH)
+        _write_stamp(STAMP_PATH, source_hash(extra_flags))
     return out
+
+
+def _write_stamp(path: Path, text: str) -> None:
+    tmp = path.with_suffix(".stamp.tmp")
+    tmp.write_text(text)
+    os.replace(tmp, path)
+
+
+# ---------------------------------------------------------------- host extension
+def host_hash() -> str:
+    """Sources and flags, and the PyTorch and Python whose object layouts are compiled in."""
+    import torch
+
+    h = hashlib.sha256()
+    for f in (HOST_SOURCE, SRC_DIR / "fo_api.h"):
+        h.update(f.read_bytes())
+    h.update(" ".join([*HOST_FLAGS, torch.__version__, sys.version]).encode())
+    return h.hexdigest()
+
+
+def host_is_current() -> bool:
+    return HOST_PATH.exists() and HOST_STAMP_PATH.exists() and HOST_STAMP_PATH.read_text().strip() == host_hash()
+
+
+def build_host(force: bool = False, verbose: bool = False) -> Path:
+    """Compile ``csrc/fo_host.cpp`` into ``_lib/_fo_host.so``; returns its path."""
+    if not force and host_is_current():
+        return HOST_PATH
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+
+    cxx = os.environ.get("CXX") or shutil.which("g++")
+    if cxx is None:
+        raise RuntimeError(f"no C++ compiler: cannot build {HOST_PATH.name} (set CXX, or ship a prebuilt _lib/)")
+    cuda_home = Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
+    includes = [*cpp_extension.include_paths(), sysconfig.get_paths()["include"], str(cuda_home / "include")]
+    with _build_lock(LIB_DIR):
+        if not force and host_is_current():
+            return HOST_PATH
+        fd, tmp = tempfile.mkstemp(prefix="_fo_host.", suffix=".so.tmp", dir=str(LIB_DIR))
+        os.close(fd)
+        try:
+            cmd = [cxx, *HOST_FLAGS, f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"]
+            for d in includes:
+                cmd += ["-isystem", d]
+            cmd += [str(HOST_SOURCE), "-o", tmp]
+            for d in cpp_extension.library_paths():
+                cmd += ["-L", d]
+            cmd += ["-lc10", "-ltorch_cpu", "-ltorch_python", "-lc10_cuda"]
+            if verbose:
+                print(" ".join(cmd), flush=True)
+            r = subprocess.run(cmd, capture_output=True, text=True)
+            if r.returncode != 0:
+                raise RuntimeError(f"{cxx} failed on {HOST_SOURCE.name}:\n{r.stdout}\n{r.stderr}")
+            os.chmod(tmp, 0o755)
+            os.replace(tmp, HOST_PATH)
+        finally:
+            if os.path.exists(tmp):
+                os.unlink(tmp)
+        _write_stamp(HOST_STAMP_PATH, host_hash())
+    return HOST_PATH
 
 
 if __name__ == "__main__":
     path = build(force="--force" in sys.argv, verbose=True)
     print(f"built {path}")
+    print(f"built {build_host(force='--force' in sys.argv, verbose=True)}")

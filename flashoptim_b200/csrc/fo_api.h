@@ -83,9 +83,10 @@ int fo_get_step_variant(void);
 // different paces.  A tuning knob; the built-in default is what measured best.
 void fo_set_staged_rounds(int rounds);
 int fo_get_staged_rounds(void);
-// Optional: a zeroed device uint32 (of the current device) in which a kernel sets a bit
-// when one of its bounded waits ran out (1: producer, 2: consumer of the staged kernels).
-int fo_set_step_status(void* device_word);
+// Optional: two zeroed uint32, in memory that the current device can store to (pinned host memory
+// lets the host look without a copy), which a kernel sets when one of its bounded waits ran out:
+// words[0] = 1 from a producer, words[1] = 2 from a consumer of the staged kernels.
+int fo_set_step_status(void* words);
 
 // Multi-tensor fused steps.  `segs` / `chunk_begin` are HOST pointers when
 // n_seg <= FO_MAX_INLINE_SEGS and `table_on_device` is 0 (the table then

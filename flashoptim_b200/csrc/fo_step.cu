@@ -176,10 +176,10 @@ extern "C" int fo_chunk_elems(void) { return fo::kChunk; }
 
 extern "C" void fo_set_step_variant(int variant) { fo::g_step_variant = variant; }
 extern "C" int fo_get_step_variant(void) { return fo::g_step_variant; }
-extern "C" int fo_set_step_status(void* device_word) {
+extern "C" int fo_set_step_status(void* words) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return (int)cudaErrorInvalidDevice;
-  fo::g_status[dev] = static_cast<unsigned int*>(device_word);
+  fo::g_status[dev] = static_cast<unsigned int*>(words);
   return 0;
 }
 

@@ -89,7 +89,7 @@ __device__ __forceinline__ void staged_body(const StepParams& P, const Hyper& H,
     for (int c = blockIdx.x; c < w.total; c += gridDim.x, ++j) {
       const int s = j % kStages;
       if (j >= kStages && !mbar_wait(&empty[s], ((j / kStages) - 1) & 1)) {
-        if (P.status) atomicOr(P.status, 1u);
+        report_timeout(P.status, 0);
         return;
       }
       w.seek(c);
@@ -127,7 +127,7 @@ __device__ __forceinline__ void staged_body(const StepParams& P, const Hyper& H,
     // one verdict per warp: at the deadline lanes may disagree, and the group shuffles in
     // store_unit need all 32 lanes
     if (!__all_sync(kFullMask, mbar_wait(&full[s], (j / kStages) & 1))) {
-      if (P.status && lane == 0) atomicOr(P.status, 2u);
+      if (lane == 0) report_timeout(P.status, 1);
       return;
     }
     Regs r;

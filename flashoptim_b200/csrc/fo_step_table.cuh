@@ -33,9 +33,17 @@ struct StepParams {
   const int32_t* chunk_begin;  // device table (null when inline)
   int n_seg;
   int total_chunks;
-  unsigned int* status;  // optional device word where a kernel records a wait that ran out
+  unsigned int* status;  // optional pair of words where a kernel records a wait that ran out
   InlineTable inl;
 };
+
+// Records a wait that ran out in word `who` (0: producer, 1: consumer).  Plain stores: the words
+// usually live in host memory, where read-modify-write operations of a GPU are not atomic.
+__device__ __forceinline__ void report_timeout(unsigned int* status, int who) {
+  if (!status) return;
+  reinterpret_cast<volatile unsigned int*>(status)[who] = 1u << who;
+  __threadfence_system();
+}
 
 // Walks the chunk list of one CTA: chunk c belongs to the segment s with
 // chunk_begin[s] <= c < chunk_begin[s + 1]; a CTA visits chunks in increasing

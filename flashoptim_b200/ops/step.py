@@ -44,69 +44,64 @@ def _launch(name: str, fn, *args) -> int:
 
 def launch_count() -> int:
     """Number of fused step kernels launched by this process so far."""
-    return _launches
+    from . import host
+
+    mod = host.loaded()
+    return _launches + (mod.launches() if mod is not None else 0)
 
 
 class StepKernelError(RuntimeError):
     """A bounded wait inside a step kernel ran out (the update of that launch is incomplete)."""
 
 
-_status: dict[int, torch.Tensor] = {}
+# Per device: two pinned words in which its step kernels record a wait that ran out (0: producer,
+# 1: consumer).  Kernels store to them over the bus, which happens only on a timeout, so that the
+# host can look at them after every step without a copy, an event or a wait.  (A device word read
+# back through a pinned copy and an event cost 2.4 us of the stream and about 15 us of the host
+# per step.)
+_status: dict[int, memoryview] = {}
+_status_keep: list[torch.Tensor] = []
 
 
-def _ensure_status(device: torch.device) -> None:
-    """Give the kernels of ``device`` a word to report a wait that ran out."""
-    idx = device.index if device.index is not None else torch.cuda.current_device()
+def _ensure_status(device) -> None:
+    """Give the kernels of ``device`` (or its index) the words to report a wait that ran out."""
+    idx = device if isinstance(device, int) else device.index
+    if idx is None:
+        idx = torch.cuda.current_device()
     if idx not in _status:
-        t = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", idx))
+        t = torch.zeros(2, dtype=torch.int32).pin_memory()
         with torch.cuda.device(idx):
             native.check(native.load().fo_set_step_status(t.data_ptr()), "fo_set_step_status")
-        _status[idx] = t
+        _status_keep.append(t)
+        _status[idx] = memoryview(t.numpy())
+
+
+def _raise_if_set(idx: int, words: memoryview) -> None:
+    code = words[0] | words[1]
+    if code:
+        words[0] = words[1] = 0
+        raise StepKernelError(f"cuda:{idx}: step kernel wait timed out (code {code})")
 
 
 def check_kernel_status(device: Optional[torch.device] = None) -> None:
     """Synchronise and raise :class:`StepKernelError` if a step kernel reported a timeout."""
-    for idx, t in list(_status.items()):
+    for idx, words in list(_status.items()):
         if device is not None and device.index not in (None, idx):
             continue
-        code = int(t.item())
-        if code:
-            t.zero_()
-            raise StepKernelError(f"cuda:{idx}: step kernel wait timed out (code {code})")
-
-
-_polls: dict[int, tuple[torch.Tensor, "torch.cuda.Event"]] = {}
-_poll_hosts: dict[int, torch.Tensor] = {}  # one pinned word per device, reused by every poll
+        torch.cuda.synchronize(idx)
+        _raise_if_set(idx, words)
 
 
 def poll_kernel_status() -> None:
-    """Non-blocking form of :func:`check_kernel_status`, meant to be called once per step.
+    """Non-blocking form of :func:`check_kernel_status`, called once per step.
 
-    Each call looks at the copy of the status word that the previous call requested (if that
-    copy has arrived) and requests a fresh one on the current stream, so the host never waits
-    for the device.  A bounded wait that ran out inside a step kernel (the warps concerned
-    skipped their chunks, i.e. part of that update is missing) therefore raises
-    :class:`StepKernelError` one or two calls late.  Call :func:`check_kernel_status` where the
-    answer must be current, e.g. before a checkpoint is written."""
-    for idx, t in list(_status.items()):
-        pending = _polls.get(idx)
-        if pending is not None:
-            host, event = pending
-            if not event.query():
-                continue  # still in flight: ask again next time
-            del _polls[idx]
-            code = int(host.item())
-            if code:
-                t.zero_()
-                raise StepKernelError(f"cuda:{idx}: step kernel wait timed out (code {code})")
-        with torch.cuda.device(idx):
-            host = _poll_hosts.get(idx)
-            if host is None:
-                host = _poll_hosts[idx] = torch.empty(1, dtype=torch.int32).pin_memory()
-            host.copy_(t, non_blocking=True)
-            event = torch.cuda.Event()
-            event.record()
-        _polls[idx] = (host, event)
+    The host never waits for the device: a bounded wait that ran out inside a step kernel (the
+    warps concerned skipped their chunks, i.e. part of that update is missing) raises
+    :class:`StepKernelError` at the first call after the kernel has said so, usually one or two
+    steps late.  Call :func:`check_kernel_status` where the answer must be current, e.g. before a
+    checkpoint is written."""
+    for idx, words in tuple(_status.items()):
+        _raise_if_set(idx, words)
 
 
 def set_step_variant(variant: int) -> None:

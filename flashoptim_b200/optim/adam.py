@@ -14,6 +14,9 @@ from .base import FlashOptimizer
 from .state import QuantizedTensorSpec
 
 
+_MOMENTS = ("exp_avg", "exp_avg_sq")
+
+
 class FlashAdam(FlashOptimizer):
     """Adam with L2 regularisation folded into the gradient (``torch.optim.Adam``
     semantics).  States: ``exp_avg`` (int8, companded) and ``exp_avg_sq`` (uint8,
@@ -89,6 +92,10 @@ class FlashAdam(FlashOptimizer):
             wd *= hparams["lr"] / hparams["initial_lr"] if self._decouple_lr else hparams["lr"]
         return wd
 
+    def _native_step_args(self, hparams):
+        lr, (beta1, beta2) = hparams["lr"], hparams["betas"]
+        return _MOMENTS, True, (lr, beta1, beta2, hparams["eps"], self._folded_weight_decay(hparams), self._decoupled)
+
     def _eager_step(self, param, grad, errors, param_state, hparams) -> None:
         m_state, v_state = param_state["exp_avg"], param_state["exp_avg_sq"]
         p32, m32, v32 = oracle.adam_math(
@@ -127,7 +134,7 @@ class FlashAdam(FlashOptimizer):
                 step=step,
                 decoupled=self._decoupled,
             )
-            rows = pack_rows(bucket, ("exp_avg", "exp_avg_sq"))
+            rows = pack_rows(bucket, _MOMENTS)
             if peer is None:
                 table = self._table((group_index, device, dtype, err, quantized, len(bucket)), device)
                 launch_adam(table, rows, dtype, err, quantized, hyper)

@@ -17,6 +17,9 @@ What differs by design:
 * ``step()`` is one kernel launch per (parameter group, dtype/ECC/quantisation
   combination) instead of one per tensor: all tensors of a bucket are described
   by a segment table and updated by a persistent multi-tensor sm_100a kernel.
+* The walk over a group's parameters that builds this table runs in native code
+  (``csrc/fo_host.cpp``); the Python walk below it serves CPU tensors,
+  ``fused=False`` and whatever the native one hands back.
 * Without a GPU everything still works: CPU tensors take the PyTorch
   formulation of the same numerics (the reference raises
   ``NotImplementedError``, ``flashoptim/optimizers.py:484-493``).
@@ -28,6 +31,7 @@ What differs by design:
 from __future__ import annotations
 
 import abc
+import importlib
 import math
 import os
 import warnings
@@ -36,10 +40,14 @@ from typing import Any, Callable, Iterable, Literal, Optional, cast
 import torch
 import torch.nn as nn
 
-from ..ops import oracle
+from ..ops import host, oracle
 from ..ops.quant import compute_ecc_bits, maxabs, reconstruct_fp32_param
 from ..ops.step import SegmentTable, poll_kernel_status
 from .state import MaybeQuantizedTensor, QuantizedTensorSpec
+
+# Step hooks that apply to every optimizer of the process; where torch does not show them, assume some.
+_torch_optimizer = importlib.import_module(torch.optim.Optimizer.__module__)
+_global_step_hooks = [getattr(_torch_optimizer, f"_global_optimizer_{when}_hooks", (None,)) for when in ("pre", "post")]
 
 _VALID_MASTER_WEIGHT_BITS = (None, 24, 32)
 _BITS_TO_BYTES = {None: 0, 24: 3, 32: 4}
@@ -130,6 +138,10 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
         self._transient_state: dict[int, dict[str, Any]] = {}
         # device segment tables of the fused launches, keyed by bucket
         self._tables: dict[Any, SegmentTable] = {}
+        # native walk over the CUDA parameters of a group, created by the first step
+        self._walker: Any = None
+        # ids of the parameters whose state was looked over by _ensure_state_initialized
+        self._state_ready: set[int] = set()
         # parameters already updated during this backward by a kernel fused with the
         # gradient collective (see flashoptim_b200.parallel); the next step()/step_param()
         # skips them once
@@ -215,6 +227,12 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
         With ``peer`` (a :class:`flashoptim_b200.parallel.symm.PeerGradients`) the
         gradient entries are byte offsets into the ranks' symmetric buffers and the
         kernels average them over NVLink while updating."""
+
+    def _native_step_args(self, hparams: dict[str, Any]) -> Optional[tuple[tuple[str, ...], bool, tuple]]:
+        """What the native walk needs to know about a group: names of the moments in kernel
+        order, whether the rule is Adam's, and its scalars (``csrc/fo_host.cpp``, ``adam_hyper``
+        and ``momentum_hyper``).  None: this class is stepped by the Python walk only."""
+        return None
 
     def _initial_value_for_state_var(self, param: torch.Tensor, key: str) -> torch.Tensor:
         del key
@@ -304,10 +322,9 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
         if self._check_numerics and self._transient_state.get(id(p), {}).get("maxabs") is None:
             self._recompute_stats_for_param(p)
         state = self.state[p]
-        ready = self.__dict__.setdefault("_state_ready", set())
-        if state and id(p) in ready:
+        if state and id(p) in self._state_ready:
             return  # created (or loaded) earlier; an emptied state is rebuilt below
-        ready.add(id(p))
+        self._state_ready.add(id(p))
         p_local = local_tensor(p)
         quantize = hparams.get("quantize", self._quantize)
         # states start at zero unless a subclass says otherwise; zero states are two memsets,
@@ -351,6 +368,28 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
                 return i
         return -1
 
+    def _native_step_group(self, params: list[torch.Tensor], group: dict[str, Any], group_index: int) -> bool:
+        """:meth:`_step_group` in native code.  False: nothing was changed, walk in Python."""
+        if not self._fused or not params or not params[0].is_cuda:
+            return False
+        args = self._native_step_args(group)
+        if args is None:
+            return False
+        if self._walker is None:
+            self._walker = host.load().Walker()
+        keys, adam, scalars = args
+        listeners = self._local_update_listeners
+        done = self._walker.step(
+            self, params, self.state, self._state_ready, self._peer_stepped, group, group_index, keys, adam,
+            (group["lr"], group["master_bytewidth"]) if self._check_numerics else None, bool(listeners), scalars)
+        if done is False:
+            return False
+        if listeners and done:
+            for fn in listeners:
+                fn(done)
+        return True
+
+    @torch.no_grad()
     def _step_group(self, params: list[torch.Tensor], group: dict[str, Any], group_index: int) -> None:
         """Update ``params`` (all in ``group``).  State is created for every one of
         them; those without a gradient are otherwise left alone."""
@@ -399,7 +438,6 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
             for fn in self._local_update_listeners:
                 fn(updated)
 
-    @torch.no_grad()
     def step_param(self, p: torch.Tensor, group: Optional[dict[str, Any]] = None) -> None:
         """Update one parameter from its ``.grad`` (used by gradient-release hooks).
 
@@ -409,15 +447,32 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
         """
         if group is None:
             group = self._find_group(p)
-        self._step_group([p], group, self._group_index(group))
+        index = self._group_index(group)
+        if not self._native_step_group([p], group, index):
+            self._step_group([p], group, index)
 
-    @torch.no_grad()
     def step(self, closure: Optional[Callable] = None) -> Optional[torch.Tensor]:
+        # torch wraps the step() of every optimizer class in a profiler annotation and its step
+        # hooks, which costs 9 us of a call that otherwise takes about as long.  This one (marked
+        # as wrapped already, below) takes that route only when somebody profiles or has
+        # registered a hook; a subclass with a step() of its own is wrapped by torch as usual.
+        mod = host.loaded()
+        if type(self).step is not FlashOptimizer.step or (
+            mod is not None and not mod.observed()
+            and not self._optimizer_step_pre_hooks and not self._optimizer_step_post_hooks
+            and not any(_global_step_hooks)
+        ):
+            return self._step(closure)
+        return _observed_step(self, closure)
+
+    step.hooked = True
+
+    def _step(self, closure: Optional[Callable] = None) -> Optional[torch.Tensor]:
         if self._gradient_release:
             warnings.warn(
                 "gradient release is active: the gradient hooks already update the parameters during "
                 "backward, so optimizer.step() does nothing.",
-                stacklevel=2,
+                stacklevel=3,
             )
             return None
         loss = None
@@ -425,14 +480,17 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
             with torch.enable_grad():
                 loss = closure()
         for gi, group in enumerate(self.param_groups):
-            self._step_group(group["params"], group, gi)
-        for fn in self._post_step_callbacks:
-            fn()
-        if self._fused and torch.cuda.is_available():
-            # a bounded wait that ran out inside a step kernel means part of an update is
-            # missing; reported here without waiting for the device, one or two steps late
-            # (ops.step.check_kernel_status() gives the current answer, e.g. before a checkpoint)
-            poll_kernel_status()
+            params = group["params"]
+            if not self._native_step_group(params, group, gi):
+                self._step_group(params, group, gi)
+        if self._post_step_callbacks:
+            with torch.no_grad():
+                for fn in self._post_step_callbacks:
+                    fn()
+        # a bounded wait that ran out inside a step kernel means part of an update is
+        # missing; reported here without waiting for the device, one or two steps late
+        # (ops.step.check_kernel_status() gives the current answer, e.g. before a checkpoint)
+        poll_kernel_status()
         return loss
 
     def _refuse_second_fused_update(self, p: torch.Tensor) -> None:
@@ -644,6 +702,7 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
         self._tables.clear()
         self._transient_state.clear()
         self.__dict__.setdefault("_state_ready", set()).clear()
+        self.__dict__.setdefault("_walker", None)
         opt_state = cast(dict[torch.Tensor, Any], state["state"])
         for group in cast(list[dict[str, Any]], state["param_groups"]):
             for param in group["params"]:
@@ -702,3 +761,7 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
                 width = local_param.element_size() + state["error_bits"].element_size()
                 state["error_bits"] = compute_ecc_bits(local_value, local_param, master_bytewidth=width)
         self._tables.clear()
+
+
+# step() with torch's profiler annotation and step hooks around it
+_observed_step = torch.optim.Optimizer.profile_hook_step(FlashOptimizer._step)

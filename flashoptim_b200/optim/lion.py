@@ -66,6 +66,10 @@ class FlashLion(FlashOptimizer):
             lion=True,
         )
 
+    def _native_step_args(self, hparams):
+        h = self._hyper(hparams)
+        return ("exp_avg",), False, (h.lr, h.mom_coef, h.update_coef, h.weight_decay, h.decoupled, h.lion, h.nesterov)
+
     def _eager_step(self, param, grad, errors, param_state, hparams) -> None:
         if errors is not None and errors.dtype not in (torch.int8, torch.int16):
             raise ValueError("Errors needs to be int8 or int16")

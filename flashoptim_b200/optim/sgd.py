@@ -76,6 +76,11 @@ class FlashSGD(FlashOptimizer):
             decoupled=self._decoupled,
         )
 
+    def _native_step_args(self, hparams):
+        h = self._hyper(hparams)
+        keys = ("momentum_buffer",) if h.mom_coef != 0.0 else ()
+        return keys, False, (h.lr, h.mom_coef, h.update_coef, h.weight_decay, h.decoupled, h.lion, h.nesterov)
+
     def _eager_step(self, param, grad, errors, param_state, hparams) -> None:
         h = self._hyper(hparams)
         use_mom = h.mom_coef != 0.0

@@ -1,0 +1,115 @@
+"""The native walk over a parameter group against the Python walk: same kernels, so same bits."""
+
+import copy
+
+import pytest
+import torch
+import torch.nn as nn
+
+import flashoptim_b200 as fo
+from flashoptim_b200.ops import step as fo_step
+
+pytestmark = pytest.mark.gpu
+
+
+def _state_tensors(opt):
+    out = []
+    for group in opt.param_groups:
+        for p in group["params"]:
+            for key, v in sorted(opt.state[p].items()):
+                parts = [v] if isinstance(v, torch.Tensor) else [v.quantized, v.scales] if v.is_quantized() else [v.data]
+                out += [(key, t.cpu()) for t in parts]
+            out.append(("param", p.detach().cpu()))
+    return out
+
+
+def _make(cls, kw, dtypes, count, seed=0):
+    g = torch.Generator().manual_seed(seed)
+    params = []
+    for i in range(count):
+        n = (1, 33, 4097, 64, 31, 8192)[i % 6]
+        params.append(nn.Parameter(torch.randn(n, generator=g).to(dtypes[i % len(dtypes)]).cuda()))
+    params[1].requires_grad_(False)
+    params.append(nn.Parameter(torch.zeros(0, dtype=dtypes[0], device="cuda")))
+    return params, cls([dict(params=params[:count // 2]), dict(params=params[count // 2:], lr=0.02)], lr=0.01, **kw)
+
+
+def _grads(params, seed, skip):
+    g = torch.Generator().manual_seed(seed)
+    for i, p in enumerate(params):
+        grad = torch.randn(p.shape, generator=g).to(p.dtype).cuda()
+        p.grad = grad if p.requires_grad and i not in skip else None
+
+
+@pytest.mark.parametrize("cls,kw", [
+    (fo.FlashAdamW, {}), (fo.FlashAdam, dict(weight_decay=0.1, quantize=False, master_weight_bits=32)),
+    (fo.FlashLion, dict(weight_decay=0.1, master_weight_bits=32)), (fo.FlashSGDW, dict(momentum=0.9, nesterov=True)),
+    (fo.FlashSGD, {}), (fo.FlashAdamW, dict(check_numerics=True)),
+])
+@pytest.mark.parametrize("count", [6, 44])  # table inside the kernel parameters, table on the device
+def test_native_walk_equals_python_walk(cls, kw, count, monkeypatch):
+    dtypes = (torch.bfloat16, torch.bfloat16, torch.float32, torch.float16)
+    results = []
+    for native in (True, False):
+        params, opt = _make(cls, kw, dtypes, count)
+        if not native:
+            monkeypatch.setattr(opt, "_native_step_group", lambda *a: False)
+        for it in range(4):
+            # other parameters lack a gradient each time (step counts diverge), addresses move
+            _grads(params, 10 + it, {it, it + 3})
+            if it == 2:  # a state that was replaced, and one that was emptied
+                opt.state[params[0]] = copy.copy(opt.state[params[0]])
+                opt.state[params[4]] = {}
+            n0 = fo_step.launch_count()
+            opt.step()
+            assert fo_step.launch_count() > n0
+        assert native == (opt._walker is not None)
+        torch.cuda.synchronize()
+        results.append(_state_tensors(opt))
+    assert len(results[0]) == len(results[1])
+    for (ka, a), (kb, b) in zip(*results):
+        assert ka == kb and torch.equal(a, b), ka
+
+
+def test_step_param_skips_what_a_collective_updated_once():
+    p = nn.Parameter(torch.randn(100, device="cuda").bfloat16())
+    opt = fo.FlashAdamW([p], lr=0.1)
+    p.grad = torch.ones_like(p)
+    opt._peer_stepped.add(id(p))
+    before = p.detach().clone()
+    opt.step_param(p)
+    assert torch.equal(p, before) and not opt._peer_stepped
+    opt.step_param(p, opt.param_groups[0])
+    assert not torch.equal(p, before) and opt.state[p]["step"].item() == 1
+
+
+def test_refusals_come_from_the_python_walk():
+    p = nn.Parameter(torch.randn(8, 8, device="cuda").bfloat16())
+    opt = fo.FlashAdamW([p], lr=0.1)
+    p.grad = torch.ones(8, 8, device="cuda", dtype=torch.bfloat16).t()[:, ::1].t().t()
+    with pytest.raises(RuntimeError, match="contiguous gradient"):
+        opt.step()
+    p.grad = torch.ones_like(p)
+    opt.step()
+    opt.state[p]["exp_avg"]._quantized = torch.zeros(63, dtype=torch.int8, device="cuda")
+    with pytest.raises(ValueError, match="63 codes"):
+        opt.step()
+
+
+def test_hooks_and_profiler_still_see_the_step():
+    p = nn.Parameter(torch.randn(100, device="cuda").bfloat16())
+    opt = fo.FlashAdamW([p], lr=0.1)
+    p.grad = torch.ones_like(p)
+    opt.step()
+    calls = []
+    h = opt.register_step_pre_hook(lambda *a: calls.append("pre"))
+    opt.register_step_post_hook(lambda *a: calls.append("post"))
+    opt.step()
+    assert calls == ["pre", "post"]
+    h.remove()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as prof:
+        opt.step()
+    assert any("Optimizer.step#FlashAdamW" in e.key for e in prof.key_averages())
+    sched = torch.optim.lr_scheduler.StepLR(opt, 1)
+    opt.step()
+    sched.step()
