@@ -69,11 +69,18 @@ __device__ __forceinline__ void store_raw8(const Raw8<T>& r, T* base, int cnt, b
 
 // A segment is "vector safe" when every base pointer is 16-byte aligned; unit
 // offsets are multiples of 8 elements, so alignment then holds for every unit.
-__device__ __forceinline__ bool seg_vector_safe(const FoSeg& s) {
-  uintptr_t a = reinterpret_cast<uintptr_t>(s.p) | reinterpret_cast<uintptr_t>(s.g) |
-                reinterpret_cast<uintptr_t>(s.ecc) | reinterpret_cast<uintptr_t>(s.s0) |
-                reinterpret_cast<uintptr_t>(s.s1);
+// The gradient is looked at on its own: as a view of a communication bucket it starts wherever
+// the tensor before it ended, while parameter and states keep the allocator's alignment.
+__device__ __forceinline__ bool seg_state_vector_safe(const FoSeg& s) {
+  uintptr_t a = reinterpret_cast<uintptr_t>(s.p) | reinterpret_cast<uintptr_t>(s.ecc) |
+                reinterpret_cast<uintptr_t>(s.s0) | reinterpret_cast<uintptr_t>(s.s1);
   return (a & 15) == 0;
+}
+__device__ __forceinline__ bool seg_grad_vector_safe(const FoSeg& s) {
+  return (reinterpret_cast<uintptr_t>(s.g) & 15) == 0;
+}
+__device__ __forceinline__ bool seg_vector_safe(const FoSeg& s) {
+  return seg_state_vector_safe(s) && seg_grad_vector_safe(s);
 }
 
 // Loads everything except the gradient.

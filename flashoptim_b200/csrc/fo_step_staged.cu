@@ -23,44 +23,172 @@
 
 namespace fo {
 
-// Ring depth and CTAs per SM.  On the 291-tensor Llama-3-8B list 4 stages x 3 CTAs
-// (9 chunks = 131 KB in flight per SM) measured best or within noise of the best for
-// every kernel; deeper rings with 2 CTAs win on a single huge tensor but not on the
-// list.  -DFO_STAGES / -DFO_STAGED_CTAS_PER_SM override both for tuning builds.
-template <int kErr>
-struct StageConfig {
-#if defined(FO_STAGES) && defined(FO_STAGED_CTAS_PER_SM)
-  static constexpr int kStages = FO_STAGES, kCtasPerSm = FO_STAGED_CTAS_PER_SM;
-#else
-  static constexpr int kStages = 4;
-  static constexpr int kCtasPerSm = 3;
-#endif
-};
-constexpr int kConsumerThreads = 256;
+// A consumer thread owns kSpan = 16 consecutive elements of a chunk, half a quantisation group:
+// the group's absmax takes one shuffle, codes move as 16-byte vectors, and what a thread spends per
+// chunk outside the arithmetic (barrier, addresses, constants, scales) is shared by 16 elements.
+// These kernels are bound by instruction issue and, through it, by the power cap (the clock falls
+// to 1.63 of 1.965 GHz within 0.1 s).
+constexpr int kSpan = 16;
+constexpr int kStagedChunk = kChunk;  // elements; the chunk prefix is shared with the register path
+constexpr int kConsumerThreads = kStagedChunk / kSpan;
 constexpr int kConsumerWarps = kConsumerThreads / 32;
 constexpr int kStagedThreads = kConsumerThreads + 32;
-constexpr int kStagedChunk = kConsumerThreads * kUnit;  // must equal kChunk of the table
-static_assert(kStagedChunk == kChunk, "staged kernels share the chunk prefix of the register path");
+
+// Ring depth and CTAs per SM.  -DFO_STAGES / -DFO_STAGED_CTAS_PER_SM override both for tuning builds.
+#ifndef FO_STAGES
+#define FO_STAGES 3
+#endif
+#ifndef FO_STAGED_CTAS_PER_SM
+#define FO_STAGED_CTAS_PER_SM 4
+#endif
+template <int kErr>
+struct StageConfig {
+  static constexpr int kStages = FO_STAGES;
+  static constexpr int kCtasPerSm = FO_STAGED_CTAS_PER_SM;
+};
 
 template <int kErr, int kStates>
 struct StageLayout {
   static constexpr int kP = 0;
-  static constexpr int kG = kP + kStagedChunk * 2;
-  static constexpr int kEcc = kG + kStagedChunk * 2;
+  static constexpr int kEcc = kP + kStagedChunk * 2;
   static constexpr int kQ0 = kEcc + kStagedChunk * kErr;
   static constexpr int kQ1 = kQ0 + kStagedChunk;
   static constexpr int kS0 = kQ0 + kStagedChunk * kStates;
   static constexpr int kS1 = kS0 + (kStagedChunk / kGroup) * 2;
-  static constexpr int kBytes = kS0 + kStates * (kStagedChunk / kGroup) * 2;
-  static constexpr int kStride = (kBytes + 127) / 128 * 128;
+  // gradient last: 16 bytes more when it does not start on a 16-byte boundary
+  static constexpr int kG = kS0 + kStates * (kStagedChunk / kGroup) * 2;
+  static constexpr int kBytes = kG + kStagedChunk * 2;
+  static constexpr int kStride = (kBytes + 16 + 127) / 128 * 128;
 };
 
 // A chunk goes through the copy engine when it is a full block of a segment whose
-// streams (including the scale vectors) are 16-byte aligned.
+// streams (including the scale vectors) are 16-byte aligned.  The gradient may start anywhere:
+// the copy then begins at the 16-byte boundary below it and ends at the one above its last byte
+// (both inside the 16-byte blocks that the gradient itself touches), and the consumers shift.
+// Element-wise global loads instead cost three times the whole update (0.79 against 0.26 ms for
+// 108 M fp16 elements).
 __device__ __forceinline__ bool chunk_is_staged(const ChunkWalker& w, int c) {
   const uintptr_t a = reinterpret_cast<uintptr_t>(w.S.s0s) | reinterpret_cast<uintptr_t>(w.S.s1s);
   const int64_t base = (int64_t)(c - w.seg_begin) * kStagedChunk;
   return w.vec && (a & 15) == 0 && base + kStagedChunk <= w.S.n;
+}
+
+// 32 bytes of the narrow parameter: one 256-bit store where the address allows.
+__device__ __forceinline__ void st32_narrow(void* p, const uint4& lo, const uint4& hi) {
+  if ((reinterpret_cast<uintptr_t>(p) & 31) == 0) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(lo.x), "r"(lo.y), "r"(lo.z),
+                 "r"(lo.w), "r"(hi.x), "r"(hi.y), "r"(hi.z), "r"(hi.w)
+                 : "memory");
+  } else {
+    st16(p, lo);
+    st16(static_cast<char*>(p) + 16, hi);
+  }
+}
+
+// 32 bytes that start kWord words and `bits` (0 or 16) bits into three 16-byte vectors.
+template <int kWord>
+__device__ __forceinline__ void shift_words(const uint32_t (&w)[12], int bits, uint4 (&out)[2]) {
+  uint32_t o[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) o[i] = __funnelshift_r(w[i + kWord], w[i + kWord + 1], bits);
+  out[0] = make_uint4(o[0], o[1], o[2], o[3]);
+  out[1] = make_uint4(o[4], o[5], o[6], o[7]);
+}
+// A span of a gradient whose first element lies `skew` bytes (2 ... 14) behind `src`.
+__device__ __forceinline__ void load_skewed(const unsigned char* src, int skew, uint4 (&out)[2]) {
+  uint32_t w[12];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const uint4 x = *reinterpret_cast<const uint4*>(src + i * 16);
+    w[4 * i] = x.x, w[4 * i + 1] = x.y, w[4 * i + 2] = x.z, w[4 * i + 3] = x.w;
+  }
+  const int bits = (skew & 3) * 8;
+  switch (skew >> 2) {
+    case 0: shift_words<0>(w, bits, out); break;
+    case 1: shift_words<1>(w, bits, out); break;
+    case 2: shift_words<2>(w, bits, out); break;
+    default: shift_words<3>(w, bits, out); break;
+  }
+}
+
+// One span out of shared memory, updated and stored.
+template <typename T, int kErr, int kStates, typename Hyper, typename Update>
+__device__ __forceinline__ void staged_span(const FoSeg& S, int64_t chunk_base, const unsigned char* st,
+                                            uint64_t* empty_bar, const Hyper& H, Update update) {
+  using L = StageLayout<kErr, kStates>;
+  const int t = threadIdx.x;
+  Raw8<T> rp[2];
+  uint4 rg[2], ecc[2], q[2];
+  float sc[2];
+  const int skew = (int)(reinterpret_cast<uintptr_t>(S.g) & 15);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) rp[h].v = *reinterpret_cast<const uint4*>(st + L::kP + t * 32 + h * 16);
+  if (skew == 0) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) rg[h] = *reinterpret_cast<const uint4*>(st + L::kG + t * 32 + h * 16);
+  } else {
+    load_skewed(st + L::kG + t * 32, skew, rg);
+  }
+  if constexpr (kErr == 1) {
+    const uint4 e = *reinterpret_cast<const uint4*>(st + L::kEcc + t * 16);
+    ecc[0] = make_uint4(e.x, e.y, 0, 0);
+    ecc[1] = make_uint4(e.z, e.w, 0, 0);
+  } else if constexpr (kErr == 2) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) ecc[h] = *reinterpret_cast<const uint4*>(st + L::kEcc + t * 32 + h * 16);
+  }
+#pragma unroll
+  for (int k = 0; k < kStates; ++k) {
+    q[k] = *reinterpret_cast<const uint4*>(st + (k == 0 ? L::kQ0 : L::kQ1) + t * 16);
+    sc[k] = __half2float(*reinterpret_cast<const __half*>(st + (k == 0 ? L::kS0 : L::kS1) + (t >> 1) * 2));
+  }
+  __syncwarp();
+  if ((t & 31) == 0) mbar_arrive(empty_bar);  // this warp holds its spans in registers now
+
+  float2 m[2][4], v[2][4];
+  uint4 pn[2], en[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    float2 p[4], g[4], back[4], res[4];
+    unpack8<T>(rp[h], p);
+    Raw8<T> raw_g;
+    raw_g.v = rg[h];
+    unpack8<T>(raw_g, g);
+    if constexpr (kErr != 0) {
+      float2 c[4];
+      ecc_codes_scaled<T, kErr>(ecc[h], c);
+      ecc_apply8<T>(p, c);
+    }
+    dequant_softsign8(h == 0 ? make_uint2(q[0].x, q[0].y) : make_uint2(q[0].z, q[0].w), sc[0], m[h]);
+    if constexpr (kStates == 2)
+      dequant_sqrt8(h == 0 ? make_uint2(q[1].x, q[1].y) : make_uint2(q[1].z, q[1].w), sc[1], v[h]);
+    update(p, g, m[h], v[h], H);
+    Raw8<T> r;
+    pack8<T>(p, r, back);
+    pn[h] = r.v;
+    if constexpr (kErr == 1) {
+      ecc_residual8<T, 1>(p, back, res);
+      const uint2 c = round_to_bytes(res);
+      if (h == 0) en[0].x = c.x, en[0].y = c.y;
+      else en[0].z = c.x, en[0].w = c.y;
+    } else if constexpr (kErr == 2) {
+      ecc_residual8<T, 2>(p, back, res);
+      en[h] = round_to_shorts(res);
+    }
+  }
+  const int64_t base = chunk_base + t * kSpan;
+  st32_narrow(static_cast<char*>(S.p) + base * 2, pn[0], pn[1]);
+  if constexpr (kErr == 1) st16(static_cast<char*>(S.ecc) + base, en[0]);
+  else if constexpr (kErr == 2) st32_narrow(static_cast<char*>(S.ecc) + base * 2, en[0], en[1]);
+  uint4 codes;
+  const float a0 = quant_softsign16(m, codes);
+  st16(static_cast<char*>(S.s0) + base, codes);
+  if ((t & 1) == 0) static_cast<__half*>(S.s0s)[base >> 5] = __float2half_rn(a0);
+  if constexpr (kStates == 2) {
+    const float a1 = quant_sqrt16_pre(v, codes);
+    st16(static_cast<char*>(S.s1) + base, codes);
+    if ((t & 1) == 0) static_cast<__half*>(S.s1s)[base >> 5] = __float2half_rn(a1);
+  }
 }
 
 template <typename T, int kErr, int kStates, typename Hyper, typename Update>
@@ -78,91 +206,80 @@ __device__ __forceinline__ void staged_body(const StepParams& P, const Hyper& H,
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  __syncthreads();
+  ChunkWalker w(P);  // its barrier also publishes the mbarriers
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int s = 0;           // ring position and the parity of its current round
+  uint32_t parity = 0;
   if (warp == kConsumerWarps) {
     // ---------------------------------------------------------------- producer
-    if (lane != 0) return;
-    ChunkWalker w(P);
-    int j = 0;
-    for (int c = blockIdx.x; c < w.total; c += gridDim.x, ++j) {
-      const int s = j % kStages;
-      if (j >= kStages && !mbar_wait(&empty[s], ((j / kStages) - 1) & 1)) {
+    if (lane != 0) return;  // a whole warp walking along costs 2 % of the time under the power cap
+    int round = 0;
+    for (int c = blockIdx.x; c < w.total; c += gridDim.x) {
+      if (round > 0 && !mbar_wait(&empty[s], parity ^ 1)) {
         report_timeout(P.status, 0);
+        // the consumers of stage s never came; the other stages' copies must have landed before
+        // this CTA may end
+        for (int k = 0; k < kStages; ++k)
+          if (k != s) mbar_wait(&full[k], k < s ? parity : parity ^ 1);
         return;
       }
       w.seek(c);
       if (!chunk_is_staged(w, c)) {
         mbar_arrive(&full[s]);
-        continue;
+      } else {
+        const int64_t base = (int64_t)(c - w.seg_begin) * kStagedChunk;
+        unsigned char* st = smem + s * L::kStride;
+        const char* g = static_cast<const char*>(w.S.g) + base * 2;
+        const uint32_t skew = (uint32_t)(reinterpret_cast<uintptr_t>(g) & 15), more = skew ? 16 : 0;
+        constexpr uint32_t kScaleBytes = (kStagedChunk / kGroup) * 2;
+        mbar_arrive_expect_tx(&full[s], L::kBytes + more);
+        bulk_load(st + L::kP, static_cast<const char*>(w.S.p) + base * 2, kStagedChunk * 2, &full[s]);
+        bulk_load(st + L::kG, g - skew, kStagedChunk * 2 + more, &full[s]);
+        if constexpr (kErr > 0)
+          bulk_load(st + L::kEcc, static_cast<const char*>(w.S.ecc) + base * kErr, kStagedChunk * kErr, &full[s]);
+        bulk_load(st + L::kQ0, static_cast<const char*>(w.S.s0) + base, kStagedChunk, &full[s]);
+        bulk_load(st + L::kS0, static_cast<const char*>(w.S.s0s) + (base >> 5) * 2, kScaleBytes, &full[s]);
+        if constexpr (kStates == 2) {
+          bulk_load(st + L::kQ1, static_cast<const char*>(w.S.s1) + base, kStagedChunk, &full[s]);
+          bulk_load(st + L::kS1, static_cast<const char*>(w.S.s1s) + (base >> 5) * 2, kScaleBytes, &full[s]);
+        }
       }
-      const int64_t base = (int64_t)(c - w.seg_begin) * kStagedChunk;
-      unsigned char* st = smem + s * L::kStride;
-      mbar_arrive_expect_tx(&full[s], L::kBytes);
-      bulk_load(st + L::kP, static_cast<const char*>(w.S.p) + base * 2, kStagedChunk * 2, &full[s]);
-      bulk_load(st + L::kG, static_cast<const char*>(w.S.g) + base * 2, kStagedChunk * 2, &full[s]);
-      if constexpr (kErr > 0)
-        bulk_load(st + L::kEcc, static_cast<const char*>(w.S.ecc) + base * kErr, kStagedChunk * kErr, &full[s]);
-      bulk_load(st + L::kQ0, static_cast<const char*>(w.S.s0) + base, kStagedChunk, &full[s]);
-      bulk_load(st + L::kS0, static_cast<const char*>(w.S.s0s) + (base >> 5) * 2, (kStagedChunk / kGroup) * 2,
-                &full[s]);
-      if constexpr (kStates == 2) {
-        bulk_load(st + L::kQ1, static_cast<const char*>(w.S.s1) + base, kStagedChunk, &full[s]);
-        bulk_load(st + L::kS1, static_cast<const char*>(w.S.s1s) + (base >> 5) * 2, (kStagedChunk / kGroup) * 2,
-                  &full[s]);
-      }
+      if (++s == kStages) s = 0, parity ^= 1, round = 1;
     }
     return;
   }
 
   // ------------------------------------------------------------------ consumers
-  ChunkWalker w(P);
-  int j = 0;
-  for (int c = blockIdx.x; c < w.total; c += gridDim.x, ++j) {
-    const int s = j % kStages;
+  for (int c = blockIdx.x; c < w.total; c += gridDim.x) {
     w.seek(c);
-    const bool staged = chunk_is_staged(w, c);
-    const int64_t base = (int64_t)(c - w.seg_begin) * kStagedChunk + (int64_t)threadIdx.x * kUnit;
-    // one verdict per warp: at the deadline lanes may disagree, and the group shuffles in
-    // store_unit need all 32 lanes
-    if (!__all_sync(kFullMask, mbar_wait(&full[s], (j / kStages) & 1))) {
+    const int64_t chunk_base = (int64_t)(c - w.seg_begin) * kStagedChunk;
+    // one verdict per warp: at the deadline lanes may disagree, and the group shuffles need all
+    // 32 lanes
+    if (!__all_sync(kFullMask, mbar_wait(&full[s], parity))) {
       if (lane == 0) report_timeout(P.status, 1);
       return;
     }
-    Regs r;
-    if (staged) {
-      const unsigned char* st = smem + s * L::kStride;
-      r.cnt = kUnit;
-      r.p.v = *reinterpret_cast<const uint4*>(st + L::kP + threadIdx.x * 16);
-      r.g.v = *reinterpret_cast<const uint4*>(st + L::kG + threadIdx.x * 16);
-      r.ecc = make_uint4(0, 0, 0, 0);
-      if constexpr (kErr == 1) {
-        const uint2 e = *reinterpret_cast<const uint2*>(st + L::kEcc + threadIdx.x * 8);
-        r.ecc.x = e.x;
-        r.ecc.y = e.y;
-      } else if constexpr (kErr == 2) {
-        r.ecc = *reinterpret_cast<const uint4*>(st + L::kEcc + threadIdx.x * 16);
-      }
-      r.q[0] = *reinterpret_cast<const uint2*>(st + L::kQ0 + threadIdx.x * 8);
-      r.sc[0] = __half2float(*reinterpret_cast<const __half*>(st + L::kS0 + (threadIdx.x >> 2) * 2));
-      if constexpr (kStates == 2) {
-        r.q[1] = *reinterpret_cast<const uint2*>(st + L::kQ1 + threadIdx.x * 8);
-        r.sc[1] = __half2float(*reinterpret_cast<const __half*>(st + L::kS1 + (threadIdx.x >> 2) * 2));
-      }
+    if (chunk_is_staged(w, c)) {
+      staged_span<T, kErr, kStates>(w.S, chunk_base, smem + s * L::kStride, &empty[s], H, update);
     } else {
-      load_unit_state(r, w.S, base, w.vec);
-      load_unit_grad(r, w.S, base, w.vec);
-    }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&empty[s]);  // this warp holds its units in registers now
-    float2 p[4], g[4], m[4], v[4];
+      if (lane == 0) mbar_arrive(&empty[s]);  // nothing was staged
+#pragma unroll 1
+      for (int u = 0; u < kSpan / kUnit; ++u) {
+        const int64_t base = chunk_base + (int64_t)(u * kConsumerThreads + threadIdx.x) * kUnit;
+        Regs r;
+        load_unit_state(r, w.S, base, w.vec);
+        load_unit_grad(r, w.S, base, w.vec_grad);
+        float2 p[4], g[4], m[4], v[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) m[i] = v[i] = make_float2(0.f, 0.f);
-    unpack8<T>(r.g, g);
-    widen_unit(r, p, m, v);
-    update(p, g, m, v, H);
-    store_unit(r, w.S, base, w.vec, p, m, v);
+        for (int i = 0; i < 4; ++i) m[i] = v[i] = make_float2(0.f, 0.f);
+        unpack8<T>(r.g, g);
+        widen_unit(r, p, m, v);
+        update(p, g, m, v, H);
+        store_unit(r, w.S, base, w.vec, p, m, v);
+      }
+    }
+    if (++s == kStages) s = 0, parity ^= 1;
   }
 }
 
