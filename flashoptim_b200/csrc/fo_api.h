@@ -106,6 +106,21 @@ int fo_quantize(const void* x, int dtype, void* q, void* scales, int64_t n, int 
 int fo_dequantize(const void* q, const void* scales, float* out, int64_t n, int is_signed, int do_sqrt,
                   int softsign, void* stream);
 
+// The same for a list of tensors (host memory, read before the call returns), 12 to a launch.
+//   quantise:    src values, dst codes, dst2 scales
+//   dequantise:  src codes, aux scales, dst values (`out_dtype` fp32 or bf16, rounded from fp32)
+typedef struct {
+  const void* src;
+  const void* aux;
+  void* dst;
+  void* dst2;
+  int64_t n;
+} FoConvRow;
+int fo_quantize_many(const FoConvRow* rows, int n_rows, int dtype, int is_signed, int do_sqrt, int softsign,
+                     void* stream);
+int fo_dequantize_many(const FoConvRow* rows, int n_rows, int out_dtype, int is_signed, int do_sqrt, int softsign,
+                       void* stream);
+
 // Master-weight split: narrow (bf16/fp16) + int8/int16 codes <-> fp32 (exact).
 int fo_ecc_decode(const void* narrow, int dtype, const void* ecc, int err_bytes, float* out, int64_t n,
                   void* stream);

@@ -15,9 +15,11 @@
 namespace fo {
 
 constexpr int kQThreads = 256;
-// Register budgets (launch bounds) that measured best on B200: 32 registers (8 CTAs per SM) for
-// the quantiser and dequantiser, 40 (6 CTAs, nothing spilled) for the master-weight kernels.
-constexpr int kQuantMinBlocks = 8;
+// Register budgets (launch bounds) that measured best at 2^28 elements: 40 registers (6 CTAs per SM)
+// for the quantiser (bf16, companded: 151 us; 158 with 48, 172 with 64), 32 (8 CTAs) for the
+// dequantiser (to bf16: 172 us; 193 with 40, 205 with 48), 40 for the master-weight kernels.
+constexpr int kQuantMinBlocks = 6;
+constexpr int kDequantMinBlocks = 8;
 constexpr int kEccMinBlocks = 6;
 
 // ---------------------------------------------------------------- memory access
@@ -45,12 +47,6 @@ __device__ __forceinline__ void st32(void* p, const Words8& v) {
                "r"(v.w[3]), "r"(v.w[4]), "r"(v.w[5]), "r"(v.w[6]), "r"(v.w[7])
                : "memory");
 }
-
-// The quantiser and dequantiser give a thread one unit of 8 consecutive elements per iteration
-// (four lanes form a group of 32) and move it with vector accesses when the tensor's base
-// address allows and the unit is whole: 32 bytes for fp32 (two 16-byte requests when the unit
-// is only 16-byte aligned), 16 for 2-byte and 8 for 1-byte elements.  Tails and unaligned
-// tensors go element by element.  The arithmetic per element is the same in both paths.
 
 template <typename T>
 __device__ __forceinline__ float load_as_float(const T* p, int64_t i) {
@@ -99,114 +95,243 @@ __device__ __forceinline__ void load8f(const T* p, int64_t base, int64_t n, bool
     for (int i = 0; i < kUnit; ++i) v[i] = base + i < n ? load_as_float(p, base + i) : 0.0f;
   }
 }
-__device__ __forceinline__ void store8f(float* p, int64_t base, int64_t n, bool vec, const float (&v)[kUnit]) {
-  if (vec && base + kUnit <= n) {
+// ---------------------------------------------------------------- lists of tensors
+//
+// A call covers a list of tensors (the states of a whole checkpoint): their addresses travel in
+// the kernel parameters, kMaxRows to a launch, and CTAs take chunks of kConvChunk elements off the
+// concatenated list.  A CTA's chunk numbers only grow, so it steps through the rows.
+constexpr int kSpan = 16;  // elements per thread and chunk
+constexpr int kConvChunk = kQThreads * kSpan;
+constexpr int kMaxRows = 12;  // 0.6 KB of parameters; the 2.8 KB of 64 rows made a small launch 1 us longer
+struct ConvBatch {
+  FoConvRow rows[kMaxRows];
+  int32_t begin[kMaxRows + 1];  // first chunk of each row
+  int total;
+};
+__device__ __forceinline__ void seek_row(const ConvBatch& B, int c, int& r) {
+  while (c >= B.begin[r + 1]) ++r;
+}
+__device__ __forceinline__ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+// 16 elements of any supported float type -> fp32 (exact widening); zero beyond n.
+template <typename T>
+__device__ __forceinline__ void load_span(const T* p, int64_t base, int64_t n, float2 (&v)[8]) {
+  constexpr int kWords = sizeof(T) * 4;
+  if (aligned16(p) && base + kSpan <= n) {
+    uint32_t w[kWords];
     if (aligned32(p + base)) {
-      Words8 o;
 #pragma unroll
-      for (int i = 0; i < kUnit; ++i) o.w[i] = __float_as_uint(v[i]);
-      st32(p + base, o);
+      for (int k = 0; k < kWords / 8; ++k) {
+        const Words8 a = ldg32(reinterpret_cast<const uint32_t*>(p + base) + 8 * k);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) w[8 * k + i] = a.w[i];
+      }
     } else {
-      st16(p + base, make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3])));
-      st16(p + base + 4,
-           make_uint4(__float_as_uint(v[4]), __float_as_uint(v[5]), __float_as_uint(v[6]), __float_as_uint(v[7])));
+#pragma unroll
+      for (int k = 0; k < kWords / 4; ++k) {
+        const uint4 a = ldg16(reinterpret_cast<const uint32_t*>(p + base) + 4 * k);
+        w[4 * k] = a.x; w[4 * k + 1] = a.y; w[4 * k + 2] = a.z; w[4 * k + 3] = a.w;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if constexpr (sizeof(T) == 4)
+        v[i] = make_float2(__uint_as_float(w[2 * i]), __uint_as_float(w[2 * i + 1]));
+      else if constexpr (std::is_same<T, __half>::value)
+        v[i] = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+      else
+        v[i] = make_float2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
     }
   } else {
 #pragma unroll
-    for (int i = 0; i < kUnit; ++i)
-      if (base + i < n) p[base + i] = v[i];
-  }
-}
-// 8 one-byte integers (two's complement in the low bits of c[i]).
-template <typename E>
-__device__ __forceinline__ void store8i(E* p, int64_t base, int64_t n, bool vec, const int (&c)[kUnit]) {
-  static_assert(sizeof(E) == 1, "8-bit codes only");
-  if (vec && base + kUnit <= n) {
-    uint2 o;
-    o.x = (c[0] & 0xff) | ((c[1] & 0xff) << 8) | ((c[2] & 0xff) << 16) | ((uint32_t)(c[3] & 0xff) << 24);
-    o.y = (c[4] & 0xff) | ((c[5] & 0xff) << 8) | ((c[6] & 0xff) << 16) | ((uint32_t)(c[7] & 0xff) << 24);
-    st8(p + base, o);
-  } else {
-#pragma unroll
-    for (int i = 0; i < kUnit; ++i)
-      if (base + i < n) p[base + i] = (E)c[i];
-  }
-}
-template <typename E>
-__device__ __forceinline__ void load8i(const E* p, int64_t base, int64_t n, bool vec, int (&c)[kUnit]) {
-  static_assert(sizeof(E) == 1, "8-bit codes only");
-  if (vec && base + kUnit <= n) {
-    const uint2 a = ldg8(p + base);
-    const uint32_t w[2] = {a.x, a.y};
-#pragma unroll
-    for (int i = 0; i < kUnit; ++i) {
-      const uint32_t b = (w[i >> 2] >> (8 * (i & 3))) & 0xffu;
-      c[i] = std::is_signed<E>::value ? (int)(int8_t)b : (int)b;
+    for (int i = 0; i < 8; ++i) {
+      v[i].x = base + 2 * i < n ? load_as_float(p, base + 2 * i) : 0.0f;
+      v[i].y = base + 2 * i + 1 < n ? load_as_float(p, base + 2 * i + 1) : 0.0f;
     }
-  } else {
-#pragma unroll
-    for (int i = 0; i < kUnit; ++i) c[i] = base + i < n ? (int)p[base + i] : 0;
   }
 }
 
-// One thread per unit of 8 elements; four lanes form a group.
+// ---------------------------------------------------------------- quantiser
+
+// One code as the written-down formula has it: correctly rounded square root and divisions.
+template <bool kSigned, bool kSqrt, bool kSoftsign>
+__device__ __forceinline__ uint32_t exact_code(float x, float a) {
+  if (kSqrt) x = __fsqrt_rn(x);
+  float t = __fdiv_rn(x, a);
+  if (kSoftsign) t = __fdiv_rn(__fmul_rn(t, 2.0f), __fadd_rn(fabsf(t), 1.0f));
+  return (uint32_t)(int)floorf(__fadd_rn(__fmul_rn(t, kSigned ? 127.0f : 255.0f), 0.5f));
+}
+
+// A thread takes half a group: one shuffle per group maximum, 16-byte code vectors.
+//
+// The formula's two correctly rounded divisions (and square root) per element made the kernel
+// issue bound at a third of the memory bandwidth (2^28 elements, bf16: companded 357 us, sqrt domain
+// 314; now 152 and 183, 5.4 and 4.5 TB/s).  Here a code is first computed with one
+// approximate reciprocal (or square root) per element; its distance to the nearest rounding
+// boundary then says whether the formula's own rounding errors could have led to the neighbouring
+// code, and only then (about one element in 4000) the formula is evaluated.
+//   Bound, in units of 2^-24 relative to the scaled value s: approximation <= 6 with the compander
+//   (constant, its product, FMA, reciprocal 2, product) or 6 without (square root 2, reciprocal 2,
+//   two products), formula <= 4 plus half an ulp of s + 0.5.  With |s| <= 127 that is at most
+//   8e-5, with |s| <= 255 at most 1.7e-4; kNear lies above both.  NaN fails the comparison, so
+//   that everything that is not finite takes the formula too; an infinite group maximum gives
+//   zero on both ways.
+// The square root is monotonic: the root of the group maximum is the maximum of the roots.
 template <typename T, bool kSigned, bool kSqrt, bool kSoftsign>
 __global__ void __launch_bounds__(kQThreads, kQuantMinBlocks)
-    quantize_kernel(const T* __restrict__ x, uint8_t* __restrict__ q, __half* __restrict__ scales, int64_t n) {
-  const int64_t n_units = ((n + kGroup - 1) / kGroup) * (kGroup / kUnit);
-  const bool vec = aligned_for_units(x) && aligned_for_units(q);
-  for (int64_t unit = (int64_t)blockIdx.x * kQThreads + threadIdx.x; unit - threadIdx.x < n_units;
-       unit += (int64_t)gridDim.x * kQThreads) {
-    const int64_t base = unit * kUnit;
-    const bool live = unit < n_units;
-    float v[kUnit];
-    load8f(x, base, live ? n : 0, vec, v);  // zero beyond the tensor: padding cannot raise the absmax
+    quantize_kernel(const __grid_constant__ ConvBatch B) {
+  constexpr float kMax = kSigned ? 127.0f : 255.0f;
+  constexpr float kNear = kSigned ? 0x1p-13f : 0x1p-12f;
+  int r = 0;
+  for (int c = blockIdx.x; c < B.total; c += gridDim.x) {
+    seek_row(B, c, r);
+    const int64_t n = B.rows[r].n;
+    const int64_t base = (int64_t)(c - B.begin[r]) * kConvChunk + threadIdx.x * kSpan;
+    float2 x[8];
+    load_span(static_cast<const T*>(B.rows[r].src), base, n, x);  // zero beyond the tensor: padding cannot raise the absmax
     float a = 0.0f;
 #pragma unroll
-    for (int i = 0; i < kUnit; ++i) {
-      if (kSqrt) v[i] = __fsqrt_rn(v[i]);
-      a = fmaxf(a, fabsf(v[i]));
-    }
-    a = fmaxf(group_max(a), 1e-12f);
-    const float qmax = kSigned ? 127.0f : 255.0f;
-    int c[kUnit];
+    for (int i = 0; i < 8; ++i)
+      a = kSqrt ? fmaxf(a, fmaxf(x[i].x, x[i].y)) : fmaxf(a, fmaxf(fabsf(x[i].x), fabsf(x[i].y)));
+    a = fmaxf(a, __shfl_xor_sync(kFullMask, a, 1));
+    if (kSqrt) a = __fsqrt_rn(a);
+    a = fmaxf(a, 1e-12f);
+
+    constexpr float kInv = 1.0f / (2.0f * kMax);
+    // scaled by 2^-32 so that the reciprocal of the largest maxima does not underflow
+    const float k = kSoftsign ? __fmul_rn(a, kInv) : __fmul_rn(fast_rcp(a * 0x1p-32f), kMax * 0x1p-32f);
+    const float2 magic = splat2(kRoundMagic), neg1 = splat2(-1.0f);
+    uint32_t w[4];
 #pragma unroll
-    for (int i = 0; i < kUnit; ++i) {
-      float t = __fdiv_rn(v[i], a);
-      if (kSoftsign) t = __fdiv_rn(__fmul_rn(t, 2.0f), __fadd_rn(fabsf(t), 1.0f));
-      c[i] = (int)floorf(__fadd_rn(__fmul_rn(t, qmax), 0.5f));
+    for (int h = 0; h < 2; ++h) {
+      float2 s[4];
+      uint32_t z[8];
+      bool sure = true;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float2 v = x[4 * h + i];
+        if (kSqrt) v = make_float2(fast_sqrt(v.x), fast_sqrt(v.y));
+        // with the compander, MAX * 2n / (1 + |n|) for n = v / a is v / ((a + |v|) / (2 MAX))
+        const float2 f = kSoftsign ? make_float2(fast_rcp(fmaf(fabsf(v.x), kInv, k)), fast_rcp(fmaf(fabsf(v.y), kInv, k)))
+                                   : splat2(k);
+        s[i] = mul2(v, f);
+        const float2 q = add2(s[i], magic);
+        const float2 off = add2(s[i], fma2(q, neg1, magic));  // from the nearest integer
+        sure = sure && fabsf(off.x) < 0.5f - kNear && fabsf(off.y) < 0.5f - kNear;
+        z[2 * i] = __float_as_uint(q.x);
+        z[2 * i + 1] = __float_as_uint(q.y);
+      }
+      if (!sure) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float si = (i & 1) ? s[i >> 1].y : s[i >> 1].x;
+          const float xi = (i & 1) ? x[4 * h + (i >> 1)].y : x[4 * h + (i >> 1)].x;
+          const float off = __fsub_rn(si, __fsub_rn(__uint_as_float(z[i]), kRoundMagic));
+          if (!(fabsf(off) < 0.5f - kNear)) z[i] = exact_code<kSigned, kSqrt, kSoftsign>(xi, a);
+        }
+      }
+      w[2 * h] = __byte_perm(__byte_perm(z[0], z[1], 0x0040), __byte_perm(z[2], z[3], 0x0040), 0x5410);
+      w[2 * h + 1] = __byte_perm(__byte_perm(z[4], z[5], 0x0040), __byte_perm(z[6], z[7], 0x0040), 0x5410);
     }
-    if (live) {
-      if (kSigned) store8i(reinterpret_cast<int8_t*>(q), base, n, vec, c);
-      else store8i(q, base, n, vec, c);
+    uint8_t* q = static_cast<uint8_t*>(B.rows[r].dst);
+    if (base + kSpan <= n && aligned16(q)) {
+      st16(q + base, make_uint4(w[0], w[1], w[2], w[3]));
+    } else {
+#pragma unroll
+      for (int i = 0; i < kSpan; ++i)
+        if (base + i < n) q[base + i] = (uint8_t)(w[i >> 2] >> (8 * (i & 3)));
     }
-    if ((threadIdx.x & 3) == 0 && live && base < n) scales[base >> 5] = __float2half_rn(a);
+    if ((threadIdx.x & 1) == 0 && base < n) static_cast<__half*>(B.rows[r].dst2)[base >> 5] = __float2half_rn(a);
   }
 }
 
-template <bool kSigned, bool kSqrt, bool kSoftsign>
-__global__ void __launch_bounds__(kQThreads, kQuantMinBlocks)
-    dequantize_kernel(const uint8_t* __restrict__ q, const __half* __restrict__ scales, float* __restrict__ out,
-                      int64_t n) {
-  const int64_t n_units = (n + kUnit - 1) / kUnit;
-  const bool vec = aligned_for_units(q) && aligned_for_units(out);
-  for (int64_t unit = (int64_t)blockIdx.x * kQThreads + threadIdx.x; unit < n_units;
-       unit += (int64_t)gridDim.x * kQThreads) {
-    const int64_t base = unit * kUnit;
-    const float sc = __half2float(scales[base >> 5]);
-    const float qmax = kSigned ? 127.0f : 255.0f;
-    int c[kUnit];
-    if (kSigned) load8i(reinterpret_cast<const int8_t*>(q), base, n, vec, c);
-    else load8i(q, base, n, vec, c);
-    float r[kUnit];
+// ---------------------------------------------------------------- dequantiser
+
+// a / b from an approximate reciprocal of b, the product and one correction by its exact remainder
+// (Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", 1990).
+__device__ __forceinline__ float corrected_quotient(float a, float b, float rcp_b) {
+  const float q = __fmul_rn(a, rcp_b);
+  return __fmaf_rn(__fmaf_rn(-q, b, a), rcp_b, q);
+}
+// What the formula divides depends on the code alone, so that 256 codes are all there is to check:
+// equal to IEEE division for each of them (tests/test_quantizer_boundaries_gpu.py).  With IEEE
+// divisions 2^28 elements took 326-367 us (companded, to fp32), with these 213 (6.3 TB/s), with a
+// table of the values in shared memory, one copy per bank, 277.
+template <bool kSigned, bool kSoftsign>
+__device__ __forceinline__ float code_value(float c) {
+  constexpr float kMax = kSigned ? 127.0f : 255.0f;
+  const float t = corrected_quotient(c, kMax, 1.0f / kMax);
+  if (!kSoftsign) return t;
+  const float d = __fsub_rn(2.0f, fabsf(t));
+  return corrected_quotient(t, d, fast_rcp(d));
+}
+
+// An access takes the codes of 8 elements per lane, contiguous over the warp.
+template <typename T, bool kSigned, bool kSqrt, bool kSoftsign>
+__global__ void __launch_bounds__(kQThreads, kDequantMinBlocks)
+    dequantize_kernel(const __grid_constant__ ConvBatch B) {
+  constexpr int kAccesses = kSpan / kUnit;
+  int r = 0;
+  for (int c = blockIdx.x; c < B.total; c += gridDim.x) {
+    seek_row(B, c, r);
+    const int64_t n = B.rows[r].n;
+    const uint8_t* q = static_cast<const uint8_t*>(B.rows[r].src);
+    const __half* scales = static_cast<const __half*>(B.rows[r].aux);
+    T* out = static_cast<T*>(B.rows[r].dst);
+    const int64_t first = (int64_t)(c - B.begin[r]) * kConvChunk + threadIdx.x * kUnit;
+    const bool vec = (reinterpret_cast<uintptr_t>(q) & 7) == 0;
+    uint32_t w[kAccesses][2];
+    float sc[kAccesses];
 #pragma unroll
-    for (int i = 0; i < kUnit; ++i) {
-      float t = __fdiv_rn((float)c[i], qmax);
-      if (kSoftsign) t = __fdiv_rn(t, __fsub_rn(2.0f, fabsf(t)));
-      r[i] = __fmul_rn(t, sc);
-      if (kSqrt) r[i] = __fmul_rn(r[i], r[i]);
+    for (int k = 0; k < kAccesses; ++k) {
+      const int64_t base = first + k * (kQThreads * kUnit);
+      sc[k] = base < n ? __half2float(scales[base >> 5]) : 0.0f;
+      if (base + kUnit <= n && vec) {
+        const uint2 a = ldg8(q + base);
+        w[k][0] = a.x;
+        w[k][1] = a.y;
+      } else {
+        ld_partial<1, 2>(q + base, (int)min(n - base, (int64_t)kUnit), w[k]);
+      }
     }
-    store8f(out, base, n, vec, r);
+#pragma unroll
+    for (int k = 0; k < kAccesses; ++k) {
+      const int64_t base = first + k * (kQThreads * kUnit);
+      float2 x[4];
+      if (kSigned) s8_to_float(make_uint2(w[k][0], w[k][1]), x);
+      else u8_to_float(make_uint2(w[k][0], w[k][1]), x);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        x[i] = mul2(make_float2(code_value<kSigned, kSoftsign>(x[i].x), code_value<kSigned, kSoftsign>(x[i].y)), splat2(sc[k]));
+        if (kSqrt) x[i] = mul2(x[i], x[i]);
+      }
+      const int left = (int)min(n - base, (int64_t)kUnit);
+      if constexpr (sizeof(T) == 4) {
+        Words8 o;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          o.w[2 * i] = __float_as_uint(x[i].x);
+          o.w[2 * i + 1] = __float_as_uint(x[i].y);
+        }
+        if (left == kUnit && aligned32(out)) {
+          st32(out + base, o);
+        } else if (left == kUnit && aligned16(out)) {
+          st16(out + base, make_uint4(o.w[0], o.w[1], o.w[2], o.w[3]));
+          st16(out + base + 4, make_uint4(o.w[4], o.w[5], o.w[6], o.w[7]));
+        } else {
+          st_partial<4, 8>(out + base, left, o.w);
+        }
+      } else {
+        uint32_t o[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const __nv_bfloat162 b = __floats2bfloat162_rn(x[i].x, x[i].y);
+          o[i] = *reinterpret_cast<const uint32_t*>(&b);
+        }
+        if (left == kUnit && aligned16(out)) st16(out + base, make_uint4(o[0], o[1], o[2], o[3]));
+        else st_partial<2, 4>(out + base, left, o);
+      }
+    }
   }
 }
 
@@ -465,24 +590,27 @@ __global__ void __launch_bounds__(kQThreads) maxabs_kernel(const T* __restrict__
 // to round quantisation (2.7-3.2 rounds at a residency of 5-6); 24 / 32 / 48 / 128 per SM got
 // faster in that order; one unit per thread over the whole grid (no loop) was slower again for
 // five of the seven kernels.  -DFO_QUANT_BLOCKS_PER_SM=k changes the factor for tuning builds.
+// The kernels over lists, whose chunk is twice as large, cap their grids accordingly (quantiser at
+// 2^28 elements: 168 us with 16 CTAs per SM, 158 with 64, 166 with 256).
+constexpr int kListCtasPerSm = 64;
 #ifndef FO_QUANT_BLOCKS_PER_SM
 #define FO_QUANT_BLOCKS_PER_SM 128
 #endif
-static int blocks_for(int64_t units) {
+static int sm_count() {
   static int sms[64];
   int dev = 0;
   cudaGetDevice(&dev);
-  int n = 148;
-  if (dev >= 0 && dev < 64) {
-    if (sms[dev] == 0) {
-      int v = 0;
-      if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) v = 148;
-      sms[dev] = v;
-    }
-    n = sms[dev];
+  if (dev < 0 || dev >= 64) return 148;
+  if (sms[dev] == 0) {
+    int v = 0;
+    if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) v = 148;
+    sms[dev] = v;
   }
+  return sms[dev];
+}
+static int blocks_for(int64_t units) {
   int64_t b = (units + kQThreads - 1) / kQThreads;
-  const int64_t cap = (int64_t)n * FO_QUANT_BLOCKS_PER_SM;
+  const int64_t cap = (int64_t)sm_count() * FO_QUANT_BLOCKS_PER_SM;
   if (b > cap) b = cap;
   if (b < 1) b = 1;
   return (int)b;
@@ -492,34 +620,62 @@ static void launch_strided(int64_t units, cudaStream_t st, Args... args) {
   kKernel<<<blocks_for(units), kQThreads, 0, st>>>(args...);
 }
 
-template <typename T, bool kSigned, bool kSqrt>
-static void launch_quant(const void* x, void* q, void* scales, int64_t n, int softsign, cudaStream_t st) {
-  const int64_t n_units = ((n + kGroup - 1) / kGroup) * (kGroup / kUnit);
-  if (softsign)
-    launch_strided<quantize_kernel<T, kSigned, kSqrt, true>>(n_units, st, (const T*)x, (uint8_t*)q, (__half*)scales, n);
-  else
-    launch_strided<quantize_kernel<T, kSigned, kSqrt, false>>(n_units, st, (const T*)x, (uint8_t*)q, (__half*)scales, n);
-}
-template <typename T>
-static void launch_quant_t(const void* x, void* q, void* scales, int64_t n, int is_signed, int do_sqrt,
-                           int softsign, cudaStream_t st) {
-  if (is_signed) {
-    if (do_sqrt) launch_quant<T, true, true>(x, q, scales, n, softsign, st);
-    else launch_quant<T, true, false>(x, q, scales, n, softsign, st);
-  } else {
-    if (do_sqrt) launch_quant<T, false, true>(x, q, scales, n, softsign, st);
-    else launch_quant<T, false, false>(x, q, scales, n, softsign, st);
+// Cuts a list of tensors into launches of at most kMaxRows rows.
+template <typename Launch>
+static int for_batches(const FoConvRow* rows, int n_rows, Launch launch) {
+  for (int i = 0; i < n_rows;) {
+    ConvBatch B;
+    int k = 0;
+    int64_t total = 0;
+    for (; i < n_rows && k < kMaxRows; ++i) {
+      if (rows[i].n <= 0) continue;
+      const int64_t more = (rows[i].n + kConvChunk - 1) / kConvChunk;
+      if (total + more > INT32_MAX / 2) {
+        if (k == 0) return (int)cudaErrorInvalidValue;
+        break;
+      }
+      B.rows[k] = rows[i];
+      B.begin[k++] = (int32_t)total;
+      total += more;
+    }
+    if (k == 0) break;
+    for (int j = k; j <= kMaxRows; ++j) B.begin[j] = (int32_t)total;
+    B.total = (int)total;
+    const int cap = sm_count() * kListCtasPerSm;
+    launch(B, B.total < cap ? B.total : cap);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return (int)e;
   }
+  return 0;
+}
+template <auto kKernel>
+static int launch_rows(const FoConvRow* rows, int n_rows, cudaStream_t st) {
+  return for_batches(rows, n_rows, [&](const ConvBatch& B, int grid) { kKernel<<<grid, kQThreads, 0, st>>>(B); });
 }
 
-template <bool kSigned, bool kSqrt>
-static void launch_dequant(const void* q, const void* scales, float* out, int64_t n, int softsign,
-                           cudaStream_t st) {
-  const int64_t n_units = (n + kUnit - 1) / kUnit;
-  if (softsign)
-    launch_strided<dequantize_kernel<kSigned, kSqrt, true>>(n_units, st, (const uint8_t*)q, (const __half*)scales, out, n);
-  else
-    launch_strided<dequantize_kernel<kSigned, kSqrt, false>>(n_units, st, (const uint8_t*)q, (const __half*)scales, out, n);
+// Calls f with the three recipe flags as template arguments.
+template <typename F>
+static int with_recipe(int is_signed, int do_sqrt, int softsign, F f) {
+  using Y = std::true_type;
+  using N = std::false_type;
+  if (is_signed) {
+    if (do_sqrt) return softsign ? f(Y(), Y(), Y()) : f(Y(), Y(), N());
+    return softsign ? f(Y(), N(), Y()) : f(Y(), N(), N());
+  }
+  if (do_sqrt) return softsign ? f(N(), Y(), Y()) : f(N(), Y(), N());
+  return softsign ? f(N(), N(), Y()) : f(N(), N(), N());
+}
+template <typename T>
+static int quantize_rows(const FoConvRow* rows, int n_rows, int is_signed, int do_sqrt, int softsign, cudaStream_t st) {
+  return with_recipe(is_signed, do_sqrt, softsign, [&](auto a, auto b, auto c) {
+    return launch_rows<quantize_kernel<T, decltype(a)::value, decltype(b)::value, decltype(c)::value>>(rows, n_rows, st);
+  });
+}
+template <typename T>
+static int dequantize_rows(const FoConvRow* rows, int n_rows, int is_signed, int do_sqrt, int softsign, cudaStream_t st) {
+  return with_recipe(is_signed, do_sqrt, softsign, [&](auto a, auto b, auto c) {
+    return launch_rows<dequantize_kernel<T, decltype(a)::value, decltype(b)::value, decltype(c)::value>>(rows, n_rows, st);
+  });
 }
 
 // The split / merge kernels take 8 elements per thread and iteration as well (two quads).
@@ -538,31 +694,39 @@ static void launch_maxabs(const void* x, int64_t n, float* out, cudaStream_t st)
 
 }  // namespace fo
 
+extern "C" int fo_quantize_many(const FoConvRow* rows, int n_rows, int dtype, int is_signed, int do_sqrt, int softsign,
+                                void* stream) {
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  switch (dtype) {
+    case FO_BF16: return fo::quantize_rows<__nv_bfloat16>(rows, n_rows, is_signed, do_sqrt, softsign, st);
+    case FO_FP16: return fo::quantize_rows<__half>(rows, n_rows, is_signed, do_sqrt, softsign, st);
+    case FO_FP32: return fo::quantize_rows<float>(rows, n_rows, is_signed, do_sqrt, softsign, st);
+  }
+  return (int)cudaErrorInvalidValue;
+}
+
+extern "C" int fo_dequantize_many(const FoConvRow* rows, int n_rows, int out_dtype, int is_signed, int do_sqrt,
+                                  int softsign, void* stream) {
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  switch (out_dtype) {
+    case FO_FP32: return fo::dequantize_rows<float>(rows, n_rows, is_signed, do_sqrt, softsign, st);
+    case FO_BF16: return fo::dequantize_rows<__nv_bfloat16>(rows, n_rows, is_signed, do_sqrt, softsign, st);
+  }
+  return (int)cudaErrorInvalidValue;
+}
+
 extern "C" int fo_quantize(const void* x, int dtype, void* q, void* scales, int64_t n, int is_signed,
                            int do_sqrt, int softsign, void* stream) {
   if (n <= 0) return 0;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  switch (dtype) {
-    case FO_BF16: fo::launch_quant_t<__nv_bfloat16>(x, q, scales, n, is_signed, do_sqrt, softsign, st); break;
-    case FO_FP16: fo::launch_quant_t<__half>(x, q, scales, n, is_signed, do_sqrt, softsign, st); break;
-    case FO_FP32: fo::launch_quant_t<float>(x, q, scales, n, is_signed, do_sqrt, softsign, st); break;
-    default: return (int)cudaErrorInvalidValue;
-  }
-  return (int)cudaGetLastError();
+  const FoConvRow row = {x, nullptr, q, scales, n};
+  return fo_quantize_many(&row, 1, dtype, is_signed, do_sqrt, softsign, stream);
 }
 
 extern "C" int fo_dequantize(const void* q, const void* scales, float* out, int64_t n, int is_signed,
                              int do_sqrt, int softsign, void* stream) {
   if (n <= 0) return 0;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (is_signed) {
-    if (do_sqrt) fo::launch_dequant<true, true>(q, scales, out, n, softsign, st);
-    else fo::launch_dequant<true, false>(q, scales, out, n, softsign, st);
-  } else {
-    if (do_sqrt) fo::launch_dequant<false, true>(q, scales, out, n, softsign, st);
-    else fo::launch_dequant<false, false>(q, scales, out, n, softsign, st);
-  }
-  return (int)cudaGetLastError();
+  const FoConvRow row = {q, scales, out, nullptr, n};
+  return fo_dequantize_many(&row, 1, FO_FP32, is_signed, do_sqrt, softsign, stream);
 }
 
 extern "C" int fo_ecc_decode(const void* narrow, int dtype, const void* ecc, int err_bytes, float* out,
