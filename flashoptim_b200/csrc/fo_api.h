@@ -120,6 +120,13 @@ int fo_quantize_many(const FoConvRow* rows, int n_rows, int dtype, int is_signed
                      void* stream);
 int fo_dequantize_many(const FoConvRow* rows, int n_rows, int out_dtype, int is_signed, int do_sqrt, int softsign,
                        void* stream);
+//   merge:       src narrow, aux codes, dst fp32
+//   split:       src fp32, dst narrow (its rounding), dst2 codes
+//   one-byte codes as values of the narrow `dtype`, and back (a C conversion): src, dst
+int fo_ecc_decode_many(const FoConvRow* rows, int n_rows, int dtype, int err_bytes, void* stream);
+int fo_ecc_split_many(const FoConvRow* rows, int n_rows, int dtype, int err_bytes, void* stream);
+int fo_codes_to_narrow_many(const FoConvRow* rows, int n_rows, int dtype, void* stream);
+int fo_narrow_to_codes_many(const FoConvRow* rows, int n_rows, int dtype, void* stream);
 
 // Master-weight split: narrow (bf16/fp16) + int8/int16 codes <-> fp32 (exact).
 int fo_ecc_decode(const void* narrow, int dtype, const void* ecc, int err_bytes, float* out, int64_t n,

@@ -457,17 +457,36 @@ __device__ __forceinline__ float quad_code_f(const uint32_t (&w)[sizeof(E)], int
     return __fsub_rn(__uint_as_float(__byte_perm(w[i >> 1], 0x4B000000u, (i & 1) ? 0x7432u : 0x7410u)), 8421376.0f);
 }
 
+// The tiles of a warp: a CTA takes chunks off the list, warp w of it the tiles w, w + 8, ... of each.
+struct TileWalk {
+  int chunk = blockIdx.x, tile = -1;
+  int64_t base = 0;  // first element of this lane's first quad
+  __device__ __forceinline__ bool next(const ConvBatch& B, int& row) {
+    if (++tile == kConvChunk / (kQThreads * 8)) {
+      tile = 0;
+      chunk += gridDim.x;
+    }
+    if (chunk >= B.total) return false;
+    if (tile == 0) seek_row(B, chunk, row);
+    base = (int64_t)(chunk - B.begin[row]) * kConvChunk + tile * (kQThreads * 8) + (threadIdx.x >> 5) * 256 +
+           (threadIdx.x & 31) * 4;
+    return true;
+  }
+};
+
 template <typename T, typename E>
 __global__ void __launch_bounds__(kQThreads, kEccMinBlocks)
-    ecc_decode_kernel(const T* __restrict__ w, const E* __restrict__ ecc, float* __restrict__ out, int64_t n) {
+    ecc_decode_kernel(const __grid_constant__ ConvBatch B) {
   const float smax = sizeof(E) == 1 ? 127.0f : 32767.0f;
   const uint32_t flip = sizeof(E) == 1 ? 0x80808080u : 0x80008000u;
-  const bool vec = aligned_for_quads(w) && aligned_for_quads(ecc) && aligned_for_quads(out);
-  const int lane = threadIdx.x & 31;
-  const int64_t n_tiles = (n + 255) >> 8;
-  const int64_t n_warps = (int64_t)gridDim.x * (kQThreads / 32);
-  for (int64_t tile = ((int64_t)blockIdx.x * kQThreads + threadIdx.x) >> 5; tile < n_tiles; tile += n_warps) {
-    const int64_t b[2] = {tile * 256 + lane * 4, tile * 256 + 128 + lane * 4};
+  int row = 0;
+  for (TileWalk t; t.next(B, row);) {
+    const T* w = static_cast<const T*>(B.rows[row].src);
+    const E* ecc = static_cast<const E*>(B.rows[row].aux);
+    float* out = static_cast<float*>(B.rows[row].dst);
+    const int64_t n = B.rows[row].n;
+    const bool vec = aligned_for_quads(w) && aligned_for_quads(ecc) && aligned_for_quads(out);
+    const int64_t b[2] = {t.base, t.base + 128};
     uint32_t wn[2][2], wc[2][sizeof(E)];
 #pragma unroll
     for (int hf = 0; hf < 2; ++hf) {
@@ -509,21 +528,47 @@ __global__ void __launch_bounds__(kQThreads, kEccMinBlocks)
   }
 }
 
-template <typename T, typename E>
+// Rounds two fp32 values to the narrow type, packed.
+template <typename T>
+__device__ __forceinline__ uint32_t narrow_pair(float lo, float hi) {
+  if constexpr (std::is_same<T, __half>::value) {
+    const __half2 h = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
+  } else {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
+  }
+}
+
+// Correction codes of fp32 values against their narrow roundings, which are read (kSplit false:
+// aux holds them, dst takes the codes) or made here (kSplit true: dst takes them, dst2 the codes).
+// Importing fp32 weights as a rounding, its copy into the parameter and the encoding, three
+// kernels, moved 17 bytes per element where this moves 7.
+template <typename T, typename E, bool kSplit>
 __global__ void __launch_bounds__(kQThreads, kEccMinBlocks)
-    ecc_encode_kernel(const float* __restrict__ x, const T* __restrict__ w, E* __restrict__ ecc, int64_t n) {
+    ecc_encode_kernel(const __grid_constant__ ConvBatch B) {
   const float smax = sizeof(E) == 1 ? 127.0f : 32767.0f;
-  const bool vec = aligned_for_quads(x) && aligned_for_quads(w) && aligned_for_quads(ecc);
-  const int lane = threadIdx.x & 31;
-  const int64_t n_tiles = (n + 255) >> 8;
-  const int64_t n_warps = (int64_t)gridDim.x * (kQThreads / 32);
-  for (int64_t tile = ((int64_t)blockIdx.x * kQThreads + threadIdx.x) >> 5; tile < n_tiles; tile += n_warps) {
-    const int64_t b[2] = {tile * 256 + lane * 4, tile * 256 + 128 + lane * 4};
+  int row = 0;
+  for (TileWalk t; t.next(B, row);) {
+    const float* x = static_cast<const float*>(B.rows[row].src);
+    const T* w = static_cast<const T*>(kSplit ? B.rows[row].dst : B.rows[row].aux);
+    E* ecc = static_cast<E*>(kSplit ? B.rows[row].dst2 : B.rows[row].dst);
+    const int64_t n = B.rows[row].n;
+    const bool vec = aligned_for_quads(x) && aligned_for_quads(w) && aligned_for_quads(ecc);
+    const int64_t b[2] = {t.base, t.base + 128};
     uint32_t wn[2][2], wx[2][4];
 #pragma unroll
     for (int hf = 0; hf < 2; ++hf) {
-      load4raw(w, b[hf], n, vec, wn[hf]);
       load4raw(x, b[hf], n, vec, wx[hf]);
+      if constexpr (!kSplit) load4raw(w, b[hf], n, vec, wn[hf]);
+    }
+    if constexpr (kSplit) {
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+        wn[hf][0] = narrow_pair<T>(__uint_as_float(wx[hf][0]), __uint_as_float(wx[hf][1]));
+        wn[hf][1] = narrow_pair<T>(__uint_as_float(wx[hf][2]), __uint_as_float(wx[hf][3]));
+        store4raw(const_cast<T*>(w), b[hf], n, vec, wn[hf]);
+      }
     }
 #pragma unroll
     for (int hf = 0; hf < 2; ++hf) {
@@ -561,6 +606,77 @@ __global__ void __launch_bounds__(kQThreads, kEccMinBlocks)
         else o[i >> 1] |= (uint32_t)(c & 0xffff) << (16 * (i & 1));
       }
       store4raw(ecc, b[hf], n, vec, o);
+    }
+  }
+}
+
+// ---------------------------------------------------------------- one-byte codes in the parameter's dtype
+//
+// Checkpoints carry the one-byte corrections as values of the parameter's dtype.  3 bytes per
+// element, bound by memory; torch's own conversions between int8 and the 16-bit floats reach
+// 1.1 TB/s (585 and 574 us for 218 M elements).
+__device__ __forceinline__ uint32_t signed_bytes(float lo, float hi) {
+  return (uint32_t)(uint8_t) static_cast<int8_t>(lo) | (uint32_t)(uint8_t) static_cast<int8_t>(hi) << 8;
+}
+template <typename T, bool kToNarrow>
+__global__ void __launch_bounds__(kQThreads) code_cast_kernel(const __grid_constant__ ConvBatch B) {
+  constexpr int kAccesses = kSpan / kUnit;
+  int r = 0;
+  for (int c = blockIdx.x; c < B.total; c += gridDim.x) {
+    seek_row(B, c, r);
+    const int64_t n = B.rows[r].n;
+    const void* src = B.rows[r].src;
+    void* dst = B.rows[r].dst;
+    const int8_t* q = static_cast<const int8_t*>(kToNarrow ? src : dst);
+    const T* v = static_cast<const T*>(kToNarrow ? dst : src);
+    const bool vec = (reinterpret_cast<uintptr_t>(q) & 7) == 0 && aligned16(v);
+    const int64_t first = (int64_t)(c - B.begin[r]) * kConvChunk + threadIdx.x * kUnit;
+    uint32_t in[kAccesses][kToNarrow ? 2 : 4];
+#pragma unroll
+    for (int k = 0; k < kAccesses; ++k) {
+      const int64_t base = first + k * (kQThreads * kUnit);
+      const int left = (int)min(n - base, (int64_t)kUnit);
+      if constexpr (kToNarrow) {
+        if (left == kUnit && vec) {
+          const uint2 a = ldg8(q + base);
+          in[k][0] = a.x; in[k][1] = a.y;
+        } else {
+          ld_partial<1, 2>(q + base, left, in[k]);
+        }
+      } else {
+        if (left == kUnit && vec) {
+          const uint4 a = ldg16(v + base);
+          in[k][0] = a.x; in[k][1] = a.y; in[k][2] = a.z; in[k][3] = a.w;
+        } else {
+          ld_partial<2, 4>(v + base, left, in[k]);
+        }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kAccesses; ++k) {
+      const int64_t base = first + k * (kQThreads * kUnit);
+      const int left = (int)min(n - base, (int64_t)kUnit);
+      if constexpr (kToNarrow) {
+        float2 f[4];
+        s8_to_float(make_uint2(in[k][0], in[k][1]), f);
+        uint32_t o[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) o[i] = narrow_pair<T>(f[i].x, f[i].y);
+        T* out = static_cast<T*>(dst) + base;
+        if (left == kUnit && vec) st16(out, make_uint4(o[0], o[1], o[2], o[3]));
+        else st_partial<2, 4>(out, left, o);
+      } else {
+        uint32_t o[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const uint32_t a = in[k][2 * j], b = in[k][2 * j + 1];
+          o[j] = signed_bytes(narrow_bits_to_float<T>((uint16_t)a), narrow_bits_to_float<T>((uint16_t)(a >> 16))) |
+                 signed_bytes(narrow_bits_to_float<T>((uint16_t)b), narrow_bits_to_float<T>((uint16_t)(b >> 16))) << 16;
+        }
+        int8_t* out = static_cast<int8_t*>(dst) + base;
+        if (left == kUnit && vec) st8(out, make_uint2(o[0], o[1]));
+        else st_partial<1, 2>(out, left, o);
+      }
     }
   }
 }
@@ -678,14 +794,23 @@ static int dequantize_rows(const FoConvRow* rows, int n_rows, int is_signed, int
   });
 }
 
-// The split / merge kernels take 8 elements per thread and iteration as well (two quads).
-template <typename T, typename E>
-static void launch_decode(const void* narrow, const void* ecc, float* out, int64_t n, cudaStream_t st) {
-  launch_strided<ecc_decode_kernel<T, E>>((n + kUnit - 1) / kUnit, st, (const T*)narrow, (const E*)ecc, out, n);
+template <typename T, bool kSplit>
+static int encode_rows(const FoConvRow* rows, int n_rows, int err_bytes, cudaStream_t st) {
+  if (err_bytes == 1) return launch_rows<ecc_encode_kernel<T, int8_t, kSplit>>(rows, n_rows, st);
+  if (err_bytes == 2) return launch_rows<ecc_encode_kernel<T, int16_t, kSplit>>(rows, n_rows, st);
+  return (int)cudaErrorInvalidValue;
 }
-template <typename T, typename E>
-static void launch_encode(const float* x, const void* narrow, void* ecc, int64_t n, cudaStream_t st) {
-  launch_strided<ecc_encode_kernel<T, E>>((n + kUnit - 1) / kUnit, st, x, (const T*)narrow, (E*)ecc, n);
+template <bool kSplit>
+static int encode_rows_of(const FoConvRow* rows, int n_rows, int dtype, int err_bytes, cudaStream_t st) {
+  if (dtype == FO_BF16) return encode_rows<__nv_bfloat16, kSplit>(rows, n_rows, err_bytes, st);
+  if (dtype == FO_FP16) return encode_rows<__half, kSplit>(rows, n_rows, err_bytes, st);
+  return (int)cudaErrorInvalidValue;
+}
+template <typename T>
+static int decode_rows(const FoConvRow* rows, int n_rows, int err_bytes, cudaStream_t st) {
+  if (err_bytes == 1) return launch_rows<ecc_decode_kernel<T, int8_t>>(rows, n_rows, st);
+  if (err_bytes == 2) return launch_rows<ecc_decode_kernel<T, int16_t>>(rows, n_rows, st);
+  return (int)cudaErrorInvalidValue;
 }
 template <typename T>
 static void launch_maxabs(const void* x, int64_t n, float* out, cudaStream_t st) {
@@ -729,28 +854,40 @@ extern "C" int fo_dequantize(const void* q, const void* scales, float* out, int6
   return fo_dequantize_many(&row, 1, FO_FP32, is_signed, do_sqrt, softsign, stream);
 }
 
+extern "C" int fo_ecc_decode_many(const FoConvRow* rows, int n_rows, int dtype, int err_bytes, void* stream) {
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (dtype == FO_BF16) return fo::decode_rows<__nv_bfloat16>(rows, n_rows, err_bytes, st);
+  if (dtype == FO_FP16) return fo::decode_rows<__half>(rows, n_rows, err_bytes, st);
+  return (int)cudaErrorInvalidValue;
+}
+extern "C" int fo_ecc_split_many(const FoConvRow* rows, int n_rows, int dtype, int err_bytes, void* stream) {
+  return fo::encode_rows_of<true>(rows, n_rows, dtype, err_bytes, static_cast<cudaStream_t>(stream));
+}
+extern "C" int fo_codes_to_narrow_many(const FoConvRow* rows, int n_rows, int dtype, void* stream) {
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (dtype == FO_BF16) return fo::launch_rows<fo::code_cast_kernel<__nv_bfloat16, true>>(rows, n_rows, st);
+  if (dtype == FO_FP16) return fo::launch_rows<fo::code_cast_kernel<__half, true>>(rows, n_rows, st);
+  return (int)cudaErrorInvalidValue;
+}
+extern "C" int fo_narrow_to_codes_many(const FoConvRow* rows, int n_rows, int dtype, void* stream) {
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (dtype == FO_BF16) return fo::launch_rows<fo::code_cast_kernel<__nv_bfloat16, false>>(rows, n_rows, st);
+  if (dtype == FO_FP16) return fo::launch_rows<fo::code_cast_kernel<__half, false>>(rows, n_rows, st);
+  return (int)cudaErrorInvalidValue;
+}
+
 extern "C" int fo_ecc_decode(const void* narrow, int dtype, const void* ecc, int err_bytes, float* out,
                              int64_t n, void* stream) {
   if (n <= 0) return 0;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (dtype == FO_BF16 && err_bytes == 1) fo::launch_decode<__nv_bfloat16, int8_t>(narrow, ecc, out, n, st);
-  else if (dtype == FO_BF16 && err_bytes == 2) fo::launch_decode<__nv_bfloat16, int16_t>(narrow, ecc, out, n, st);
-  else if (dtype == FO_FP16 && err_bytes == 1) fo::launch_decode<__half, int8_t>(narrow, ecc, out, n, st);
-  else if (dtype == FO_FP16 && err_bytes == 2) fo::launch_decode<__half, int16_t>(narrow, ecc, out, n, st);
-  else return (int)cudaErrorInvalidValue;
-  return (int)cudaGetLastError();
+  const FoConvRow row = {narrow, ecc, out, nullptr, n};
+  return fo_ecc_decode_many(&row, 1, dtype, err_bytes, stream);
 }
 
 extern "C" int fo_ecc_encode(const float* x, const void* narrow, int dtype, void* ecc, int err_bytes,
                              int64_t n, void* stream) {
   if (n <= 0) return 0;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (dtype == FO_BF16 && err_bytes == 1) fo::launch_encode<__nv_bfloat16, int8_t>(x, narrow, ecc, n, st);
-  else if (dtype == FO_BF16 && err_bytes == 2) fo::launch_encode<__nv_bfloat16, int16_t>(x, narrow, ecc, n, st);
-  else if (dtype == FO_FP16 && err_bytes == 1) fo::launch_encode<__half, int8_t>(x, narrow, ecc, n, st);
-  else if (dtype == FO_FP16 && err_bytes == 2) fo::launch_encode<__half, int16_t>(x, narrow, ecc, n, st);
-  else return (int)cudaErrorInvalidValue;
-  return (int)cudaGetLastError();
+  const FoConvRow row = {x, narrow, ecc, nullptr, n};
+  return fo::encode_rows_of<false>(&row, 1, dtype, err_bytes, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int fo_maxabs(const void* x, int dtype, int64_t n, float* out, void* stream) {

@@ -142,6 +142,11 @@ def _declare(lib: ctypes.CDLL) -> None:
     lib.fo_ecc_decode.argtypes = [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int64, c_void_p]
     lib.fo_ecc_encode.restype = c_int
     lib.fo_ecc_encode.argtypes = [c_void_p, c_void_p, c_int, c_void_p, c_int, c_int64, c_void_p]
+    for name, n_ints in (("fo_quantize_many", 4), ("fo_dequantize_many", 4), ("fo_ecc_decode_many", 2),
+                         ("fo_ecc_split_many", 2), ("fo_codes_to_narrow_many", 1), ("fo_narrow_to_codes_many", 1)):
+        fn = getattr(lib, name)
+        fn.restype = c_int
+        fn.argtypes = [c_void_p, c_int] + [c_int] * n_ints + [c_void_p]
     lib.fo_maxabs.restype = c_int
     lib.fo_maxabs.argtypes = [c_void_p, c_int, c_int64, c_void_p, c_void_p]
     lib.fo_comm_step_chunk_elems.restype = c_int

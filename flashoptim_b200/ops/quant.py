@@ -9,7 +9,8 @@ Both produce identical bits.  API parity with the reference:
 
 from __future__ import annotations
 
-from typing import Optional
+from array import array
+from typing import Any, Optional
 
 import torch
 
@@ -20,6 +21,94 @@ from .oracle import GROUP_SIZE, MANTISSA_BITS
 def _require_group32(group_size: int) -> None:
     if group_size != GROUP_SIZE:
         raise ValueError(f"only group_size={GROUP_SIZE} is supported, got {group_size}")
+
+
+_NARROW = (torch.bfloat16, torch.float16)
+
+
+def _splits(param: torch.Tensor, error_bits: torch.Tensor) -> bool:
+    return (param.dtype in _NARROW and error_bits.dtype in (torch.int8, torch.int16)
+            and error_bits.numel() == param.numel())
+
+
+class Conversions:
+    """Conversions of many CUDA tensors, gathered and launched together: one launch per kind and
+    12 tensors instead of one per tensor.  Inputs are kept alive until :meth:`launch`."""
+
+    def __init__(self) -> None:
+        self._lists: dict[Any, tuple[list[int], list[Any]]] = {}
+
+    def _add(self, entry: str, args: tuple[int, ...], src: torch.Tensor, aux: Optional[torch.Tensor],
+             dst: torch.Tensor, dst2: Optional[torch.Tensor] = None) -> None:
+        n = dst.numel()
+        if n == 0:
+            return
+        flat, keep = self._lists.setdefault((entry, args, dst.device), ([], []))
+        flat += (src.data_ptr(), aux.data_ptr() if aux is not None else 0, dst.data_ptr(),
+                 dst2.data_ptr() if dst2 is not None else 0, n)  # struct FoConvRow
+        keep.append((src, aux, dst, dst2))
+
+    def launch(self) -> None:
+        lists, self._lists = self._lists, {}
+        for (entry, args, device), (flat, _) in lists.items():
+            rows = array("q", flat)
+            with torch.cuda.device(device):
+                rc = getattr(native.load(), entry)(rows.buffer_info()[0], len(flat) // 5, *args,
+                                                   native.stream_ptr(device))
+            native.check(rc, entry)
+
+    def quantize(self, x: torch.Tensor, signed: bool, sqrt: bool, softsign: bool) -> tuple[torch.Tensor, torch.Tensor]:
+        """:func:`quantize` of a CUDA tensor."""
+        x = x.detach()
+        if x.dtype not in native.DTYPE_CODE:
+            x = x.to(torch.float32)
+        x = x.contiguous()
+        codes = torch.empty(x.shape, dtype=torch.int8 if signed else torch.uint8, device=x.device)
+        scales = torch.empty(oracle.num_groups(x.numel()), dtype=torch.float16, device=x.device)
+        self._add("fo_quantize_many", (native.DTYPE_CODE[x.dtype], int(signed), int(sqrt), int(softsign)),
+                  x, None, codes, scales)
+        return codes, scales
+
+    def dequantize_bf16(self, codes: torch.Tensor, scales: torch.Tensor, signed: bool, sqrt: bool,
+                        softsign: bool) -> torch.Tensor:
+        """:func:`dequantize` of CUDA codes, rounded to bf16."""
+        out = torch.empty(codes.shape, dtype=torch.bfloat16, device=codes.device)
+        self._add("fo_dequantize_many", (native.FO_BF16, int(signed), int(sqrt), int(softsign)),
+                  codes.contiguous(), scales.contiguous(), out)
+        return out
+
+    def reconstruct_fp32_param(self, param: torch.Tensor, error_bits: torch.Tensor) -> torch.Tensor:
+        """:func:`reconstruct_fp32_param`; what the list kernel does not serve goes there directly."""
+        if not (param.is_cuda and error_bits.device == param.device and _splits(param, error_bits)):
+            return reconstruct_fp32_param(param, error_bits)
+        out = torch.empty(param.shape, dtype=torch.float32, device=param.device)
+        self._add("fo_ecc_decode_many", (native.DTYPE_CODE[param.dtype], error_bits.element_size()),
+                  param.detach().contiguous(), error_bits.contiguous(), out)
+        return out
+
+    def split(self, value: torch.Tensor, param: torch.Tensor, error_bits: torch.Tensor) -> Optional[torch.Tensor]:
+        """Rounds fp32 ``value`` into ``param`` and returns the correction codes (in the dtype of
+        ``error_bits``); None, with nothing done, for what the list kernel does not serve."""
+        if not (param.is_cuda and value.device == param.device and value.shape == param.shape
+                and value.dtype == torch.float32 and param.is_contiguous() and _splits(param, error_bits)):
+            return None
+        codes = torch.empty(param.shape, dtype=error_bits.dtype, device=param.device)
+        self._add("fo_ecc_split_many", (native.DTYPE_CODE[param.dtype], codes.element_size()),
+                  value.detach().contiguous(), None, param, codes)
+        return codes
+
+    def codes_as(self, codes: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
+        """``codes.to(dtype)``; between int8 and a 16-bit float type by the list kernel."""
+        if codes.dtype == torch.int8:
+            narrow, entry = dtype, "fo_codes_to_narrow_many"
+        else:
+            narrow, entry = codes.dtype, "fo_narrow_to_codes_many"
+        if not (type(codes) is torch.Tensor and codes.is_cuda and codes.is_contiguous() and narrow in _NARROW
+                and torch.int8 in (codes.dtype, dtype)):
+            return codes.to(dtype=dtype)
+        out = torch.empty(codes.shape, dtype=dtype, device=codes.device)
+        self._add(entry, (native.DTYPE_CODE[narrow],), codes.detach(), None, out)
+        return out
 
 
 def quantize(

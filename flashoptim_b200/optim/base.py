@@ -41,7 +41,7 @@ import torch
 import torch.nn as nn
 
 from ..ops import host, oracle
-from ..ops.quant import compute_ecc_bits, maxabs, reconstruct_fp32_param
+from ..ops.quant import Conversions, compute_ecc_bits, maxabs
 from ..ops.step import SegmentTable, poll_kernel_status
 from .state import MaybeQuantizedTensor, QuantizedTensorSpec
 
@@ -582,14 +582,17 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
 
     # ------------------------------------------------------------------ checkpointing
     def _state_dict_for_param(
-        self, idx: int, packed_state: dict[int, Any], hparams: dict[str, Any], param: torch.Tensor
+        self, idx: int, packed_state: dict[int, Any], hparams: dict[str, Any], param: torch.Tensor,
+        conversions: Conversions,
     ) -> dict[str, Any]:
         out = dict(packed_state[idx])  # shallow copy: self.state stays untouched
         for key in self._quantized_state_spec():
             if key in out:
                 q = out.pop(key)
                 assert isinstance(q, MaybeQuantizedTensor)
-                out.update(q.state_dict(name=key, allow_quantized=self._compress_state_dict))
+                plain = None if self._compress_state_dict else q.as_bf16(conversions)
+                out.update({key: plain} if plain is not None
+                           else q.state_dict(name=key, allow_quantized=self._compress_state_dict))
         if "error_bits" in out:
             # torch casts state tensors to the param dtype on load and FSDP wants them
             # param-shaped, so the codes are disguised as the param dtype: same width ->
@@ -600,7 +603,7 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
             if ew == pw:
                 out["error_bits"] = errs.view(dtype=param.dtype)
             elif ew == 1 and pw == 2:
-                out["error_bits"] = errs.to(dtype=param.dtype)
+                out["error_bits"] = conversions.codes_as(errs, param.dtype)
             else:
                 raise NotImplementedError(
                     f"Cannot save {ew}B error correction tensor for {pw}B parameter: state "
@@ -612,10 +615,12 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
     def state_dict(self) -> dict[str, Any]:
         d = super().state_dict()
         packed_state, packed_groups = d["state"], d["param_groups"]
+        conversions = Conversions()
         for live, saved in zip(self.param_groups, packed_groups):
             for param, idx in zip(live["params"], saved["params"]):
                 if idx in packed_state:
-                    packed_state[idx] = self._state_dict_for_param(idx, packed_state, saved, param)
+                    packed_state[idx] = self._state_dict_for_param(idx, packed_state, saved, param, conversions)
+        conversions.launch()
         return d
 
     def load_state_dict(self, state_dict: dict[str, Any]) -> None:
@@ -644,7 +649,7 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
         self._tables.clear()
 
     def _load_state_for_param(
-        self, param: torch.Tensor, pstate: dict[str, Any], hparams: dict[str, Any]
+        self, param: torch.Tensor, pstate: dict[str, Any], hparams: dict[str, Any], conversions: Conversions
     ) -> dict[str, Any]:
         specs = self._quantized_state_spec()
         new_state: dict[str, Any] = {}
@@ -660,7 +665,7 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
             if any(k == key or k.startswith(f"{key}::") for k in pstate):
                 new_state[key] = MaybeQuantizedTensor.from_state_dict(
                     pstate, name=key, try_quantize=quantize, signed=spec.signed, sqrt=spec.sqrt,
-                    softsign=spec.softsign, storage_dtype=param.dtype,
+                    softsign=spec.softsign, storage_dtype=param.dtype, conversions=conversions,
                 )
         mbw = hparams.get("master_bytewidth")
         errs = pstate.get("error_bits")
@@ -673,7 +678,7 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
         need = mbw - pw
         src_dtype = errs.dtype
         if need == 1 and errs.dtype != torch.int8:
-            errs = errs.to(dtype=torch.int8)
+            errs = conversions.codes_as(errs, torch.int8)
         elif need == 2 and errs.dtype != torch.int16:
             errs = errs.contiguous().view(dtype=torch.int16)
         if pw + oracle.DTYPE_WIDTHS[errs.dtype] != mbw:
@@ -703,8 +708,17 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
         self._transient_state.clear()
         self.__dict__.setdefault("_state_ready", set()).clear()
         self.__dict__.setdefault("_walker", None)
-        opt_state = cast(dict[torch.Tensor, Any], state["state"])
-        for group in cast(list[dict[str, Any]], state["param_groups"]):
+        conversions = Conversions()
+        try:
+            self._load_states(cast(dict[torch.Tensor, Any], state["state"]),
+                              cast(list[dict[str, Any]], state["param_groups"]), conversions)
+        finally:  # what was loaded before an error is complete
+            conversions.launch()
+
+    def _load_states(
+        self, opt_state: dict[torch.Tensor, Any], groups: list[dict[str, Any]], conversions: Conversions
+    ) -> None:
+        for group in groups:
             for param in group["params"]:
                 if param not in opt_state:
                     continue
@@ -715,7 +729,7 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
                         pstate[key] = local_tensor(val.tensor).to(device=p_local.device)
                     elif isinstance(val, torch.Tensor):
                         pstate[key] = local_tensor(val)
-                opt_state[param] = self._load_state_for_param(param, pstate, group)
+                opt_state[param] = self._load_state_for_param(param, pstate, group, conversions)
             # after loading, so the loader can tell "came with the checkpoint" from "our default"
             group.setdefault("master_bytewidth", self._master_bytewidth)
 
@@ -734,17 +748,31 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
         corrected parameters are local shards (plain tensors).
         """
         module = cast(nn.Module, model.module if hasattr(model, "module") else model)
-        out = {k: v.detach().float() for k, v in module.state_dict().items()}
+        conversions = Conversions()
+        masters = {}
         for name, param in module.named_parameters():
             state = self.state.get(param, {})
             if "error_bits" in state:
-                out[name] = reconstruct_fp32_param(local_tensor(param.detach()), state["error_bits"])
+                masters[name] = conversions.reconstruct_fp32_param(local_tensor(param.detach()), state["error_bits"])
+        out = {k: masters[k] if k in masters else v.detach().float() for k, v in module.state_dict().items()}
+        out.update(masters)
+        conversions.launch()
         return out
 
     def set_fp32_model_state_dict(self, model: nn.Module, fp32_state_dict: dict[str, torch.Tensor]) -> None:
         """Inverse of :meth:`get_fp32_model_state_dict`: write rounded weights into the
         model and the matching correction codes into the optimizer state."""
         module = cast(nn.Module, model.module if hasattr(model, "module") else model)
+        conversions = Conversions()
+        try:
+            self._set_fp32_values(module, fp32_state_dict, conversions)
+        finally:  # what was set before an error is complete
+            conversions.launch()
+        self._tables.clear()
+
+    def _set_fp32_values(
+        self, module: nn.Module, fp32_state_dict: dict[str, torch.Tensor], conversions: Conversions
+    ) -> None:
         for name, param in module.named_parameters():
             if name not in fp32_state_dict:
                 continue
@@ -755,12 +783,16 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
             local_value = local_tensor(value)
             if local_value.device != local_param.device:
                 local_value = local_value.to(local_param.device)
-            local_param.copy_(local_value.to(param.dtype))
             state = self.state.get(param, {})
+            if "error_bits" in state:
+                codes = conversions.split(local_value, local_param, state["error_bits"])
+                if codes is not None:
+                    state["error_bits"] = codes
+                    continue
+            local_param.copy_(local_value.to(param.dtype))
             if "error_bits" in state:
                 width = local_param.element_size() + state["error_bits"].element_size()
                 state["error_bits"] = compute_ecc_bits(local_value, local_param, master_bytewidth=width)
-        self._tables.clear()
 
 
 # step() with torch's profiler annotation and step hooks around it

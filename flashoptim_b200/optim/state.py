@@ -14,7 +14,7 @@ from typing import Optional
 
 import torch
 
-from ..ops.quant import dequantize, quantize
+from ..ops.quant import Conversions, dequantize, quantize
 
 
 @dataclass(frozen=True)
@@ -136,10 +136,12 @@ class MaybeQuantizedTensor:
         )
 
     # ------------------------------------------------------------------ data movement
-    def set_data(self, data: torch.Tensor) -> None:
+    def set_data(self, data: torch.Tensor, conversions: Optional[Conversions] = None) -> None:
+        """With ``conversions``, codes and scales of a CUDA tensor are there once they are launched."""
         if self._try_quantize:
             self._data = None
-            self._quantized, self._scales = quantize(
+            fn = quantize if conversions is None or not data.is_cuda else conversions.quantize
+            self._quantized, self._scales = fn(
                 data, signed=self._signed, sqrt=self._sqrt, softsign=self._softsign
             )
         else:
@@ -164,6 +166,14 @@ class MaybeQuantizedTensor:
     def _quantized_scales_key(name: str) -> str:
         return f"{name}::scales"
 
+    def as_bf16(self, conversions: Conversions) -> Optional[torch.Tensor]:
+        """The plain flavour's tensor of a quantised CUDA state, there once ``conversions`` are
+        launched; None for any other state."""
+        if not self.is_quantized() or not self.quantized.is_cuda:
+            return None
+        return conversions.dequantize_bf16(self.quantized, self.scales, signed=self._signed, sqrt=self._sqrt,
+                                           softsign=self._softsign)
+
     def state_dict(self, name: str, allow_quantized: bool = False) -> dict[str, torch.Tensor]:
         if self.is_quantized() and allow_quantized:
             return {
@@ -172,7 +182,9 @@ class MaybeQuantizedTensor:
             }
         return {name: self.materialize().to(dtype=torch.bfloat16)}
 
-    def load_state_dict(self, d: dict[str, torch.Tensor], name: str) -> None:
+    def load_state_dict(
+        self, d: dict[str, torch.Tensor], name: str, conversions: Optional[Conversions] = None
+    ) -> None:
         d = {k: v for k, v in d.items() if k == name or k.startswith(f"{name}::")}
         if name in d:
             if len(d) != 1:
@@ -180,7 +192,7 @@ class MaybeQuantizedTensor:
                     f"a checkpoint holds either '{name}' or its compressed pair, not both; found "
                     f"{sorted(d.keys())}"
                 )
-            self.set_data(d[name])
+            self.set_data(d[name], conversions)
             return
         code_dtype = torch.int8 if self._signed else torch.uint8
         self._data = None
@@ -197,8 +209,9 @@ class MaybeQuantizedTensor:
         sqrt: bool = False,
         softsign: bool = True,
         storage_dtype: torch.dtype = torch.float32,
+        conversions: Optional[Conversions] = None,
     ) -> "MaybeQuantizedTensor":
         obj = cls(None, try_quantize=try_quantize, signed=signed, sqrt=sqrt, softsign=softsign,
                   storage_dtype=storage_dtype)
-        obj.load_state_dict(d, name)
+        obj.load_state_dict(d, name, conversions)
         return obj
