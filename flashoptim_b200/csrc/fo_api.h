@@ -73,9 +73,9 @@ int fo_chunk_elems(void);
 // Number of CTAs the step kernels are launched with on `device` (<= total chunks).
 int fo_step_grid(int device);
 
-// Kernel family of the fused steps: 1 (default) streams bf16/fp16 tensors with 8-bit
-// states through shared memory with cp.async.bulk + mbarrier stages, 0 always uses the
-// register-path kernels (which also serve every other combination).
+// Kernel family of the fused steps: 1 (default) streams tensors with 8-bit states through shared
+// memory with cp.async.bulk + mbarrier stages, 0 always uses the register-path kernels (which also
+// serve every other combination).
 void fo_set_step_variant(int variant);
 int fo_get_step_variant(void);
 // Grid of the staged kernels = resident CTAs x rounds (1..1024): with more than one round the

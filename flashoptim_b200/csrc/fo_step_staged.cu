@@ -1,11 +1,11 @@
-// Bulk-copy staged variants of the fused steps (bf16 / fp16 parameters, 8-bit states).
+// Bulk-copy staged variants of the fused steps (8-bit states).
 // Same arithmetic as the reference's step kernels (flashoptim/optimizers.py:1587-1719,
 // :2256-2443); the data path below has no counterpart there.
 //
 // The register-path kernels hold at most 32 warps x 56 B of loads in flight per
 // SM and sit at about one eligible warp per scheduler.  Here a producer warp
 // streams whole chunks (parameter, gradient, correction codes, state codes and
-// their scales: 14-17 KB) into a ring of shared-memory stages with
+// their scales: 14-21 KB) into a ring of shared-memory stages with
 // cp.async.bulk (the TMA unit's untiled copy; no multicast, no tensor map),
 // completion is tracked by one mbarrier per stage, and eight consumer warps read
 // their units from shared memory, release the stage and run the same update
@@ -34,30 +34,39 @@ constexpr int kConsumerThreads = kStagedChunk / kSpan;
 constexpr int kConsumerWarps = kConsumerThreads / 32;
 constexpr int kStagedThreads = kConsumerThreads + 32;
 
-// Ring depth and CTAs per SM.  -DFO_STAGES / -DFO_STAGED_CTAS_PER_SM override both for tuning builds.
+// Ring depth and CTAs per SM.  -DFO_STAGES / -DFO_STAGED_CTAS_PER_SM override both for tuning builds
+// (-DFO_STAGES_FP32 / -DFO_STAGED_CTAS_PER_SM_FP32 for fp32 parameters, whose stages are larger).
+// AdamW, fp32, 124 M elements in 148 tensors: register path 377 us, 3 stages on 3 CTAs 377, 4 on 2
+// 366, 2 on 4 322 (6.3 TB/s): the consumers need the warps more than the copies need the depth.
 #ifndef FO_STAGES
 #define FO_STAGES 3
 #endif
 #ifndef FO_STAGED_CTAS_PER_SM
 #define FO_STAGED_CTAS_PER_SM 4
 #endif
-template <int kErr>
+#ifndef FO_STAGES_FP32
+#define FO_STAGES_FP32 2
+#endif
+#ifndef FO_STAGED_CTAS_PER_SM_FP32
+#define FO_STAGED_CTAS_PER_SM_FP32 4
+#endif
+template <typename T>
 struct StageConfig {
-  static constexpr int kStages = FO_STAGES;
-  static constexpr int kCtasPerSm = FO_STAGED_CTAS_PER_SM;
+  static constexpr int kStages = sizeof(T) == 4 ? FO_STAGES_FP32 : FO_STAGES;
+  static constexpr int kCtasPerSm = sizeof(T) == 4 ? FO_STAGED_CTAS_PER_SM_FP32 : FO_STAGED_CTAS_PER_SM;
 };
 
-template <int kErr, int kStates>
+template <typename T, int kErr, int kStates>
 struct StageLayout {
   static constexpr int kP = 0;
-  static constexpr int kEcc = kP + kStagedChunk * 2;
+  static constexpr int kEcc = kP + kStagedChunk * (int)sizeof(T);
   static constexpr int kQ0 = kEcc + kStagedChunk * kErr;
   static constexpr int kQ1 = kQ0 + kStagedChunk;
   static constexpr int kS0 = kQ0 + kStagedChunk * kStates;
   static constexpr int kS1 = kS0 + (kStagedChunk / kGroup) * 2;
   // gradient last: 16 bytes more when it does not start on a 16-byte boundary
   static constexpr int kG = kS0 + kStates * (kStagedChunk / kGroup) * 2;
-  static constexpr int kBytes = kG + kStagedChunk * 2;
+  static constexpr int kBytes = kG + kStagedChunk * (int)sizeof(T);
   static constexpr int kStride = (kBytes + 16 + 127) / 128 * 128;
 };
 
@@ -73,8 +82,8 @@ __device__ __forceinline__ bool chunk_is_staged(const ChunkWalker& w, int c) {
   return w.vec && (a & 15) == 0 && base + kStagedChunk <= w.S.n;
 }
 
-// 32 bytes of the narrow parameter: one 256-bit store where the address allows.
-__device__ __forceinline__ void st32_narrow(void* p, const uint4& lo, const uint4& hi) {
+// 32 bytes: one 256-bit store where the address allows.
+__device__ __forceinline__ void st32(void* p, const uint4& lo, const uint4& hi) {
   if ((reinterpret_cast<uintptr_t>(p) & 31) == 0) {
     asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(lo.x), "r"(lo.y), "r"(lo.z),
                  "r"(lo.w), "r"(hi.x), "r"(hi.y), "r"(hi.z), "r"(hi.w)
@@ -85,20 +94,21 @@ __device__ __forceinline__ void st32_narrow(void* p, const uint4& lo, const uint
   }
 }
 
-// 32 bytes that start kWord words and `bits` (0 or 16) bits into three 16-byte vectors.
-template <int kWord>
-__device__ __forceinline__ void shift_words(const uint32_t (&w)[12], int bits, uint4 (&out)[2]) {
-  uint32_t o[8];
+// kVecs 16-byte vectors that start kWord words and `bits` (0 or 16) bits into one more of them.
+template <int kWord, int kVecs>
+__device__ __forceinline__ void shift_words(const uint32_t (&w)[4 * kVecs + 4], int bits, uint4 (&out)[kVecs]) {
+  uint32_t o[4 * kVecs];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) o[i] = __funnelshift_r(w[i + kWord], w[i + kWord + 1], bits);
-  out[0] = make_uint4(o[0], o[1], o[2], o[3]);
-  out[1] = make_uint4(o[4], o[5], o[6], o[7]);
+  for (int i = 0; i < 4 * kVecs; ++i) o[i] = __funnelshift_r(w[i + kWord], w[i + kWord + 1], bits);
+#pragma unroll
+  for (int i = 0; i < kVecs; ++i) out[i] = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
 }
 // A span of a gradient whose first element lies `skew` bytes (2 ... 14) behind `src`.
-__device__ __forceinline__ void load_skewed(const unsigned char* src, int skew, uint4 (&out)[2]) {
-  uint32_t w[12];
+template <int kVecs>
+__device__ __forceinline__ void load_skewed(const unsigned char* src, int skew, uint4 (&out)[kVecs]) {
+  uint32_t w[4 * kVecs + 4];
 #pragma unroll
-  for (int i = 0; i < 3; ++i) {
+  for (int i = 0; i < kVecs + 1; ++i) {
     const uint4 x = *reinterpret_cast<const uint4*>(src + i * 16);
     w[4 * i] = x.x, w[4 * i + 1] = x.y, w[4 * i + 2] = x.z, w[4 * i + 3] = x.w;
   }
@@ -111,23 +121,32 @@ __device__ __forceinline__ void load_skewed(const unsigned char* src, int skew, 
   }
 }
 
+// Half h of a span.
+template <typename T, int kVecs>
+__device__ __forceinline__ Raw8<T> raw8_of(const uint4 (&span)[kVecs], int h) {
+  Raw8<T> r;
+  r.v = span[h * kVecs / 2];
+  if constexpr (sizeof(T) == 4) r.w = span[h * kVecs / 2 + 1];
+  return r;
+}
+
 // One span out of shared memory, updated and stored.
 template <typename T, int kErr, int kStates, typename Hyper, typename Update>
 __device__ __forceinline__ void staged_span(const FoSeg& S, int64_t chunk_base, const unsigned char* st,
                                             uint64_t* empty_bar, const Hyper& H, Update update) {
-  using L = StageLayout<kErr, kStates>;
+  using L = StageLayout<T, kErr, kStates>;
+  constexpr int kSpanBytes = kSpan * sizeof(T), kVecs = kSpanBytes / 16;
   const int t = threadIdx.x;
-  Raw8<T> rp[2];
-  uint4 rg[2], ecc[2], q[2];
+  uint4 rp[kVecs], rg[kVecs], ecc[2], q[2];
   float sc[2];
   const int skew = (int)(reinterpret_cast<uintptr_t>(S.g) & 15);
 #pragma unroll
-  for (int h = 0; h < 2; ++h) rp[h].v = *reinterpret_cast<const uint4*>(st + L::kP + t * 32 + h * 16);
+  for (int i = 0; i < kVecs; ++i) rp[i] = *reinterpret_cast<const uint4*>(st + L::kP + t * kSpanBytes + i * 16);
   if (skew == 0) {
 #pragma unroll
-    for (int h = 0; h < 2; ++h) rg[h] = *reinterpret_cast<const uint4*>(st + L::kG + t * 32 + h * 16);
+    for (int i = 0; i < kVecs; ++i) rg[i] = *reinterpret_cast<const uint4*>(st + L::kG + t * kSpanBytes + i * 16);
   } else {
-    load_skewed(st + L::kG + t * 32, skew, rg);
+    load_skewed(st + L::kG + t * kSpanBytes, skew, rg);
   }
   if constexpr (kErr == 1) {
     const uint4 e = *reinterpret_cast<const uint4*>(st + L::kEcc + t * 16);
@@ -146,14 +165,13 @@ __device__ __forceinline__ void staged_span(const FoSeg& S, int64_t chunk_base, 
   if ((t & 31) == 0) mbar_arrive(empty_bar);  // this warp holds its spans in registers now
 
   float2 m[2][4], v[2][4];
-  uint4 pn[2], en[2];
+  Raw8<T> pn[2];
+  uint4 en[2];
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     float2 p[4], g[4], back[4], res[4];
-    unpack8<T>(rp[h], p);
-    Raw8<T> raw_g;
-    raw_g.v = rg[h];
-    unpack8<T>(raw_g, g);
+    unpack8<T>(raw8_of<T>(rp, h), p);
+    unpack8<T>(raw8_of<T>(rg, h), g);
     if constexpr (kErr != 0) {
       float2 c[4];
       ecc_codes_scaled<T, kErr>(ecc[h], c);
@@ -163,9 +181,7 @@ __device__ __forceinline__ void staged_span(const FoSeg& S, int64_t chunk_base, 
     if constexpr (kStates == 2)
       dequant_sqrt8(h == 0 ? make_uint2(q[1].x, q[1].y) : make_uint2(q[1].z, q[1].w), sc[1], v[h]);
     update(p, g, m[h], v[h], H);
-    Raw8<T> r;
-    pack8<T>(p, r, back);
-    pn[h] = r.v;
+    pack8<T>(p, pn[h], back);
     if constexpr (kErr == 1) {
       ecc_residual8<T, 1>(p, back, res);
       const uint2 c = round_to_bytes(res);
@@ -177,9 +193,15 @@ __device__ __forceinline__ void staged_span(const FoSeg& S, int64_t chunk_base, 
     }
   }
   const int64_t base = chunk_base + t * kSpan;
-  st32_narrow(static_cast<char*>(S.p) + base * 2, pn[0], pn[1]);
+  char* out = static_cast<char*>(S.p) + base * (int)sizeof(T);
+  if constexpr (sizeof(T) == 4) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) st32(out + h * 32, pn[h].v, pn[h].w);
+  } else {
+    st32(out, pn[0].v, pn[1].v);
+  }
   if constexpr (kErr == 1) st16(static_cast<char*>(S.ecc) + base, en[0]);
-  else if constexpr (kErr == 2) st32_narrow(static_cast<char*>(S.ecc) + base * 2, en[0], en[1]);
+  else if constexpr (kErr == 2) st32(static_cast<char*>(S.ecc) + base * 2, en[0], en[1]);
   uint4 codes;
   const float a0 = quant_softsign16(m, codes);
   st16(static_cast<char*>(S.s0) + base, codes);
@@ -193,9 +215,9 @@ __device__ __forceinline__ void staged_span(const FoSeg& S, int64_t chunk_base, 
 
 template <typename T, int kErr, int kStates, typename Hyper, typename Update>
 __device__ __forceinline__ void staged_body(const StepParams& P, const Hyper& H, Update update) {
-  using L = StageLayout<kErr, kStates>;
+  using L = StageLayout<T, kErr, kStates>;
   using Regs = UnitRegs<T, kErr, kStates, true>;
-  constexpr int kStages = StageConfig<kErr>::kStages;
+  constexpr int kStages = StageConfig<T>::kStages;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ uint64_t full[kStages], empty[kStages];
 
@@ -230,12 +252,13 @@ __device__ __forceinline__ void staged_body(const StepParams& P, const Hyper& H,
       } else {
         const int64_t base = (int64_t)(c - w.seg_begin) * kStagedChunk;
         unsigned char* st = smem + s * L::kStride;
-        const char* g = static_cast<const char*>(w.S.g) + base * 2;
+        const char* g = static_cast<const char*>(w.S.g) + base * (int)sizeof(T);
         const uint32_t skew = (uint32_t)(reinterpret_cast<uintptr_t>(g) & 15), more = skew ? 16 : 0;
+        constexpr uint32_t kValueBytes = kStagedChunk * sizeof(T);
         constexpr uint32_t kScaleBytes = (kStagedChunk / kGroup) * 2;
         mbar_arrive_expect_tx(&full[s], L::kBytes + more);
-        bulk_load(st + L::kP, static_cast<const char*>(w.S.p) + base * 2, kStagedChunk * 2, &full[s]);
-        bulk_load(st + L::kG, g - skew, kStagedChunk * 2 + more, &full[s]);
+        bulk_load(st + L::kP, static_cast<const char*>(w.S.p) + base * (int)sizeof(T), kValueBytes, &full[s]);
+        bulk_load(st + L::kG, g - skew, kValueBytes + more, &full[s]);
         if constexpr (kErr > 0)
           bulk_load(st + L::kEcc, static_cast<const char*>(w.S.ecc) + base * kErr, kStagedChunk * kErr, &full[s]);
         bulk_load(st + L::kQ0, static_cast<const char*>(w.S.s0) + base, kStagedChunk, &full[s]);
@@ -297,12 +320,12 @@ struct MomentumUpdate {
 };
 
 template <typename T, int kErr>
-__global__ void __launch_bounds__(kStagedThreads, StageConfig<kErr>::kCtasPerSm)
+__global__ void __launch_bounds__(kStagedThreads, StageConfig<T>::kCtasPerSm)
     adam_staged_kernel(const __grid_constant__ StepParams P, const __grid_constant__ FoAdamHyper H) {
   staged_body<T, kErr, 2>(P, H, AdamUpdate());
 }
 template <typename T, int kErr>
-__global__ void __launch_bounds__(kStagedThreads, StageConfig<kErr>::kCtasPerSm)
+__global__ void __launch_bounds__(kStagedThreads, StageConfig<T>::kCtasPerSm)
     momentum_staged_kernel(const __grid_constant__ StepParams P, const __grid_constant__ FoMomentumHyper H) {
   staged_body<T, kErr, 1>(P, H, MomentumUpdate());
 }
@@ -319,12 +342,12 @@ __global__ void __launch_bounds__(kStagedThreads, StageConfig<kErr>::kCtasPerSm)
 static int g_staged_rounds = FO_STAGED_ROUNDS;
 constexpr int kMinChunksPerCta = 16;
 
-template <int kErr, int kStates, typename Kernel, typename Hyper>
+template <typename T, int kErr, int kStates, typename Kernel, typename Hyper>
 static int launch_staged(Kernel kernel, const StepParams& P, const Hyper& H, int sm_count, cudaStream_t st) {
-  constexpr int smem_bytes = StageConfig<kErr>::kStages * StageLayout<kErr, kStates>::kStride;
+  constexpr int smem_bytes = StageConfig<T>::kStages * StageLayout<T, kErr, kStates>::kStride;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
   if (e != cudaSuccess) return (int)e;
-  const int64_t resident = (int64_t)sm_count * StageConfig<kErr>::kCtasPerSm;
+  const int64_t resident = (int64_t)sm_count * StageConfig<T>::kCtasPerSm;
   int64_t rounds = P.total_chunks / (resident * kMinChunksPerCta);
   if (rounds > g_staged_rounds) rounds = g_staged_rounds;
   if (rounds < 1) rounds = 1;
@@ -337,18 +360,18 @@ static int launch_staged(Kernel kernel, const StepParams& P, const Hyper& H, int
 template <typename T>
 static int staged_adam_t(const StepParams& P, const FoAdamHyper& H, int err, int sms, cudaStream_t st) {
   switch (err) {
-    case 0: return launch_staged<0, 2>(adam_staged_kernel<T, 0>, P, H, sms, st);
-    case 1: return launch_staged<1, 2>(adam_staged_kernel<T, 1>, P, H, sms, st);
-    case 2: return launch_staged<2, 2>(adam_staged_kernel<T, 2>, P, H, sms, st);
+    case 0: return launch_staged<T, 0, 2>(adam_staged_kernel<T, 0>, P, H, sms, st);
+    case 1: return launch_staged<T, 1, 2>(adam_staged_kernel<T, 1>, P, H, sms, st);
+    case 2: return launch_staged<T, 2, 2>(adam_staged_kernel<T, 2>, P, H, sms, st);
   }
   return -1;
 }
 template <typename T>
 static int staged_momentum_t(const StepParams& P, const FoMomentumHyper& H, int err, int sms, cudaStream_t st) {
   switch (err) {
-    case 0: return launch_staged<0, 1>(momentum_staged_kernel<T, 0>, P, H, sms, st);
-    case 1: return launch_staged<1, 1>(momentum_staged_kernel<T, 1>, P, H, sms, st);
-    case 2: return launch_staged<2, 1>(momentum_staged_kernel<T, 2>, P, H, sms, st);
+    case 0: return launch_staged<T, 0, 1>(momentum_staged_kernel<T, 0>, P, H, sms, st);
+    case 1: return launch_staged<T, 1, 1>(momentum_staged_kernel<T, 1>, P, H, sms, st);
+    case 2: return launch_staged<T, 2, 1>(momentum_staged_kernel<T, 2>, P, H, sms, st);
   }
   return -1;
 }
@@ -358,6 +381,7 @@ int staged_adam_launch(const StepParams& P, const FoAdamHyper& H, int dtype, int
   if (!quantized) return -1;
   if (dtype == FO_BF16) return staged_adam_t<__nv_bfloat16>(P, H, err_bytes, sm_count, st);
   if (dtype == FO_FP16) return staged_adam_t<__half>(P, H, err_bytes, sm_count, st);
+  if (dtype == FO_FP32 && err_bytes == 0) return launch_staged<float, 0, 2>(adam_staged_kernel<float, 0>, P, H, sm_count, st);
   return -1;
 }
 
@@ -366,6 +390,7 @@ int staged_momentum_launch(const StepParams& P, const FoMomentumHyper& H, int dt
   if (state_mode != FO_STATE_Q8) return -1;
   if (dtype == FO_BF16) return staged_momentum_t<__nv_bfloat16>(P, H, err_bytes, sm_count, st);
   if (dtype == FO_FP16) return staged_momentum_t<__half>(P, H, err_bytes, sm_count, st);
+  if (dtype == FO_FP32 && err_bytes == 0) return launch_staged<float, 0, 1>(momentum_staged_kernel<float, 0>, P, H, sm_count, st);
   return -1;
 }
 

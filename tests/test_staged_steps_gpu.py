@@ -64,6 +64,7 @@ def _run(rows, dtype, err, n_states, variant):
 @pytest.mark.parametrize("skew", range(8))
 @pytest.mark.parametrize("dtype,err,n_states", [
     (torch.bfloat16, 1, 2), (torch.bfloat16, 0, 1), (torch.float16, 2, 2), (torch.float16, 2, 1),
+    (torch.float32, 0, 2), (torch.float32, 0, 1),
 ])
 def test_staged_equals_register_path(dtype, err, n_states, skew):
     results = []
