@@ -30,6 +30,7 @@ template <typename T, int kErr, bool kQ>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
     adam_kernel(const __grid_constant__ StepParams P, const __grid_constant__ FoAdamHyper H) {
   using Regs = UnitRegs<T, kErr, 2, kQ>;
+  grid_begin();
   ChunkWalker w(P);
   walk_chunks<Regs>(
       w,
@@ -60,6 +61,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
   constexpr int kStates = kMode == FO_STATE_NONE ? 0 : 1;
   constexpr bool kQ = kMode == FO_STATE_Q8;
   using Regs = UnitRegs<T, kErr, kStates, kQ>;
+  grid_begin();
   ChunkWalker w(P);
   walk_chunks<Regs>(
       w,
@@ -127,9 +129,8 @@ static int fill_params(StepParams& P, const FoSeg* segs, const int32_t* chunk_be
 
 template <typename T, int kErr>
 static int launch_adam_q(const StepParams& P, const FoAdamHyper& H, int quantized, int grid, cudaStream_t st) {
-  if (quantized) adam_kernel<T, kErr, true><<<grid, kThreads, 0, st>>>(P, H);
-  else adam_kernel<T, kErr, false><<<grid, kThreads, 0, st>>>(P, H);
-  return (int)cudaGetLastError();
+  return launch_overlapped(quantized ? adam_kernel<T, kErr, true> : adam_kernel<T, kErr, false>, grid, kThreads, 0, st,
+                           P, H);
 }
 template <typename T>
 static int launch_adam_e(const StepParams& P, const FoAdamHyper& H, int err, int quantized, int grid,
@@ -145,12 +146,11 @@ static int launch_adam_e(const StepParams& P, const FoAdamHyper& H, int err, int
 template <typename T, int kErr>
 static int launch_mom_m(const StepParams& P, const FoMomentumHyper& H, int mode, int grid, cudaStream_t st) {
   switch (mode) {
-    case FO_STATE_NONE: momentum_kernel<T, kErr, FO_STATE_NONE><<<grid, kThreads, 0, st>>>(P, H); break;
-    case FO_STATE_Q8: momentum_kernel<T, kErr, FO_STATE_Q8><<<grid, kThreads, 0, st>>>(P, H); break;
-    case FO_STATE_FULL: momentum_kernel<T, kErr, FO_STATE_FULL><<<grid, kThreads, 0, st>>>(P, H); break;
-    default: return (int)cudaErrorInvalidValue;
+    case FO_STATE_NONE: return launch_overlapped(momentum_kernel<T, kErr, FO_STATE_NONE>, grid, kThreads, 0, st, P, H);
+    case FO_STATE_Q8: return launch_overlapped(momentum_kernel<T, kErr, FO_STATE_Q8>, grid, kThreads, 0, st, P, H);
+    case FO_STATE_FULL: return launch_overlapped(momentum_kernel<T, kErr, FO_STATE_FULL>, grid, kThreads, 0, st, P, H);
   }
-  return (int)cudaGetLastError();
+  return (int)cudaErrorInvalidValue;
 }
 template <typename T>
 static int launch_mom_e(const StepParams& P, const FoMomentumHyper& H, int err, int mode, int grid,

@@ -228,6 +228,7 @@ __device__ __forceinline__ void staged_body(const StepParams& P, const Hyper& H,
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  grid_begin();
   ChunkWalker w(P);  // its barrier also publishes the mbarriers
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -353,8 +354,7 @@ static int launch_staged(Kernel kernel, const StepParams& P, const Hyper& H, int
   if (rounds < 1) rounds = 1;
   int64_t grid = resident * rounds;
   if (P.total_chunks < grid) grid = P.total_chunks;
-  kernel<<<(int)grid, kStagedThreads, smem_bytes, st>>>(P, H);
-  return (int)cudaGetLastError();
+  return launch_overlapped(kernel, (int)grid, kStagedThreads, smem_bytes, st, P, H);
 }
 
 template <typename T>

@@ -92,3 +92,40 @@ def test_segment_look_up_over_many_tensors(count):
         results.append(bufs)
     for a, b in zip(*results):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("variant", [0, 1])
+def test_steps_back_to_back_and_in_a_graph(variant):
+    """A step's grid may become resident while the one before it drains: without waiting in between,
+    and replayed from a graph, the steps leave what they leave one at a time."""
+    results = []
+    for how in ("apart", "together", "graph"):
+        rows, bufs, _ = _streams((1_500_017, 70_001, 33), torch.bfloat16, 1, 2, 0, seed=1)
+        table = SegmentTable(torch.device("cuda", torch.cuda.current_device()))
+        h = AdamHyper(lr=1e-3, beta1=0.9, beta2=0.999, eps=1e-8, weight_decay=1e-5, step=7, decoupled=True)
+
+        def steps(n):
+            for _ in range(n):
+                launch_adam(table, rows, torch.bfloat16, 1, True, h)
+                if how == "apart":
+                    torch.cuda.synchronize()
+
+        set_step_variant(variant)
+        try:
+            torch.cuda.synchronize()
+            if how == "graph":
+                steps(1)  # what is set up on first use is there before the capture
+                graph = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(graph):
+                    steps(3)
+                for _ in range(13):
+                    graph.replay()
+            else:
+                steps(40)
+            torch.cuda.synchronize()
+        finally:
+            set_step_variant(1)
+        results.append(bufs)
+    for other in results[1:]:
+        for a, b in zip(results[0], other):
+            assert torch.equal(a, b)
