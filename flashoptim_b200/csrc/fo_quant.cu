@@ -172,8 +172,8 @@ __device__ __forceinline__ uint32_t exact_code(float x, float a) {
 // code, and only then (about one element in 4000) the formula is evaluated.
 //   Bound, in units of 2^-24 relative to the scaled value s: approximation <= 6 with the compander
 //   (constant, its product, FMA, reciprocal 2, product) or 6 without (square root 2, reciprocal 2,
-//   two products), formula <= 4 plus half an ulp of s + 0.5.  With |s| <= 127 that is at most
-//   8e-5, with |s| <= 255 at most 1.7e-4; kNear lies above both.  NaN fails the comparison, so
+//   two products), formula <= 4 with it or 3 without, plus half an ulp of s + 0.5.  With |s| <= 127
+//   that is at most 8e-5, with |s| <= 255 at most 1.6e-4 or 1.45e-4; kNear lies above each.  NaN fails the comparison, so
 //   that everything that is not finite takes the formula too; an infinite group maximum gives
 //   zero on both ways.
 // The square root is monotonic: the root of the group maximum is the maximum of the roots.
@@ -181,7 +181,7 @@ template <typename T, bool kSigned, bool kSqrt, bool kSoftsign>
 __global__ void __launch_bounds__(kQThreads, kQuantMinBlocks)
     quantize_kernel(const __grid_constant__ ConvBatch B) {
   constexpr float kMax = kSigned ? 127.0f : 255.0f;
-  constexpr float kNear = kSigned ? 0x1p-13f : 0x1p-12f;
+  constexpr float kNear = kSigned ? 0x1p-13f : kSoftsign ? 0x1p-12f : 0x1.4p-13f;
   int r = 0;
   for (int c = blockIdx.x; c < B.total; c += gridDim.x) {
     seek_row(B, c, r);
@@ -249,21 +249,21 @@ __global__ void __launch_bounds__(kQThreads, kQuantMinBlocks)
 
 // a / b from an approximate reciprocal of b, the product and one correction by its exact remainder
 // (Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", 1990).
-__device__ __forceinline__ float corrected_quotient(float a, float b, float rcp_b) {
-  const float q = __fmul_rn(a, rcp_b);
-  return __fmaf_rn(__fmaf_rn(-q, b, a), rcp_b, q);
+__device__ __forceinline__ float2 corrected_quotient2(float2 a, float2 neg_b, float2 rcp_b) {
+  const float2 q = mul2(a, rcp_b);
+  return fma2(fma2(q, neg_b, a), rcp_b, q);
 }
 // What the formula divides depends on the code alone, so that 256 codes are all there is to check:
 // equal to IEEE division for each of them (tests/test_quantizer_boundaries_gpu.py).  With IEEE
 // divisions 2^28 elements took 326-367 us (companded, to fp32), with these 213 (6.3 TB/s), with a
 // table of the values in shared memory, one copy per bank, 277.
 template <bool kSigned, bool kSoftsign>
-__device__ __forceinline__ float code_value(float c) {
+__device__ __forceinline__ float2 code_value2(float2 c) {
   constexpr float kMax = kSigned ? 127.0f : 255.0f;
-  const float t = corrected_quotient(c, kMax, 1.0f / kMax);
+  const float2 t = corrected_quotient2(c, splat2(-kMax), splat2(1.0f / kMax));
   if (!kSoftsign) return t;
-  const float d = __fsub_rn(2.0f, fabsf(t));
-  return corrected_quotient(t, d, fast_rcp(d));
+  const float2 neg_d = make_float2(__fsub_rn(fabsf(t.x), 2.0f), __fsub_rn(fabsf(t.y), 2.0f));
+  return corrected_quotient2(t, neg_d, make_float2(fast_rcp(-neg_d.x), fast_rcp(-neg_d.y)));
 }
 
 // An access takes the codes of 8 elements per lane, contiguous over the warp.
@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(kQThreads, kDequantMinBlocks)
       else u8_to_float(make_uint2(w[k][0], w[k][1]), x);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        x[i] = mul2(make_float2(code_value<kSigned, kSoftsign>(x[i].x), code_value<kSigned, kSoftsign>(x[i].y)), splat2(sc[k]));
+        x[i] = mul2(code_value2<kSigned, kSoftsign>(x[i]), splat2(sc[k]));
         if (kSqrt) x[i] = mul2(x[i], x[i]);
       }
       const int left = (int)min(n - base, (int64_t)kUnit);
