@@ -33,10 +33,15 @@ def _splits(param: torch.Tensor, error_bits: torch.Tensor) -> bool:
 
 class Conversions:
     """Conversions of many CUDA tensors, gathered and launched together: one launch per kind and
-    12 tensors instead of one per tensor.  Inputs are kept alive until :meth:`launch`."""
+    12 tensors instead of one per tensor.  Inputs are kept alive until :meth:`launch`, which comes by
+    itself when they reach ``HELD`` bytes: they may be copies (of a checkpoint in host memory), of
+    which a loop over tensors would hold one at a time."""
+
+    HELD = 1 << 28
 
     def __init__(self) -> None:
         self._lists: dict[Any, tuple[list[int], list[Any]]] = {}
+        self._held = 0
 
     def _add(self, entry: str, args: tuple[int, ...], src: torch.Tensor, aux: Optional[torch.Tensor],
              dst: torch.Tensor, dst2: Optional[torch.Tensor] = None) -> None:
@@ -47,9 +52,13 @@ class Conversions:
         flat += (src.data_ptr(), aux.data_ptr() if aux is not None else 0, dst.data_ptr(),
                  dst2.data_ptr() if dst2 is not None else 0, n)  # struct FoConvRow
         keep.append((src, aux, dst, dst2))
+        self._held += src.numel() * src.element_size()
+        if self._held >= self.HELD:
+            self.launch()
 
     def launch(self) -> None:
         lists, self._lists = self._lists, {}
+        self._held = 0
         for (entry, args, device), (flat, _) in lists.items():
             rows = array("q", flat)
             with torch.cuda.device(device):

@@ -118,3 +118,22 @@ def test_what_the_list_kernels_do_not_serve_is_converted_all_the_same():
     with pytest.raises(ValueError, match="Expected fp32"):
         opt.set_fp32_model_state_dict(net, bad)
     assert (net.a == 1).all() and (opt.state[net.a]["error_bits"] == 0).all()
+
+
+def test_import_from_host_memory_holds_few_copies_on_the_device(monkeypatch):
+    """24 fp32 tensors of 16 MB: 384 MB if every device copy waited for one launch at the end."""
+    monkeypatch.setattr(Conversions, "HELD", 32 << 20)
+    net = nn.ParameterList([nn.Parameter(torch.zeros(1 << 22, device="cuda", dtype=torch.bfloat16)) for _ in range(24)])
+    opt = FlashAdamW(net.parameters(), lr=1e-3)
+    for p in net:
+        p.grad = torch.zeros_like(p)
+    opt.step()
+    opt.zero_grad()
+    values = {k: torch.full((1 << 22,), 1.0 + i) for i, k in enumerate(net.state_dict())}
+    torch.cuda.synchronize()
+    base = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    opt.set_fp32_model_state_dict(net, values)
+    torch.cuda.synchronize()
+    assert torch.cuda.max_memory_allocated() - base < 24 * (4 << 20) + 96 * (1 << 20)  # new codes, and the copies in hand
+    assert all((p == 1.0 + i).all() for i, p in enumerate(net))
