@@ -45,7 +45,9 @@ static int launch_overlapped(void (*kernel)(Params...), int grid, int block, siz
   cfg.stream = st;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  return (int)cudaLaunchKernelEx(&cfg, kernel, args...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+  if (e != cudaSuccess) cudaGetLastError();  // reported here, not by somebody's next check
+  return (int)e;
 }
 
 struct InlineTable {
