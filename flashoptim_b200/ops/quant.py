@@ -37,7 +37,7 @@ class Conversions:
     itself when they reach ``HELD`` bytes: they may be copies (of a checkpoint in host memory), of
     which a loop over tensors would hold one at a time."""
 
-    HELD = 1 << 28
+    HELD = 1 << 30  # at 256 MB, a load of 1.3 GB took 555 us instead of 429: its launches got too small
 
     def __init__(self) -> None:
         self._lists: dict[Any, tuple[list[int], list[Any]]] = {}
