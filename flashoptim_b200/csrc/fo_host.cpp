@@ -12,6 +12,7 @@
 // dtype, ...) is left untouched and reported to the caller, whose Python walk updates it or says
 // what is wrong with it.  It takes the place of the per-tensor launch wrappers of the reference
 // (flashoptim/optimizers.py:1535-1583, :2203-2252).
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <ATen/ATen.h>
@@ -337,6 +338,7 @@ bool prefix(Bucket& b) {
 void upload(Bucket& b) {
   const size_t n = b.rows.size(), seg_bytes = n * sizeof(FoSeg), bytes = seg_bytes + (n + 1) * sizeof(int32_t);
   if (b.dev.defined() && b.sent.size() == n && std::memcmp(b.sent.data(), b.rows.data(), seg_bytes) == 0) return;
+  b.sent.clear();  // any line below may throw; what the buffer holds is known again once all have passed
   at::Tensor staged = at::empty({(int64_t)bytes}, at::TensorOptions().dtype(at::kByte).pinned_memory(true));
   std::memcpy(staged.data_ptr(), b.rows.data(), seg_bytes);
   std::memcpy(static_cast<char*>(staged.data_ptr()) + seg_bytes, b.chunks.data(), (n + 1) * sizeof(int32_t));
@@ -347,24 +349,24 @@ void upload(Bucket& b) {
   b.sent = b.rows;
 }
 
-// Launches one bucket; 0 or a cudaError_t.
+bool on_device(const Bucket& b) { return b.rows.size() > FO_MAX_INLINE_SEGS; }
+
+// Launches one bucket, whose table is in place; 0 or a cudaError_t.
 int launch(Bucket& b, bool adam, const FoAdamHyper& ah, const FoMomentumHyper& mh) {
   c10::cuda::OptionalCUDAGuard guard(c10::Device(c10::DeviceType::CUDA, b.device));
   const int n = (int)b.rows.size();
   const FoSeg* segs = b.rows.data();
   const int32_t* chunks = b.chunks.data();
-  const bool on_device = n > FO_MAX_INLINE_SEGS;
-  if (on_device) {
-    upload(b);
+  if (on_device(b)) {
     segs = static_cast<const FoSeg*>(b.dev.data_ptr());
     chunks = reinterpret_cast<const int32_t*>(segs + n);
   }
   void* stream = c10::cuda::getCurrentCUDAStream(b.device).stream();
   const int total = b.chunks[n];
   if (g_nvtx) nvtxRangePushA(adam ? "fo_adam_step" : "fo_momentum_step");
-  const int rc = adam ? g_api.adam_step(segs, chunks, n, total, on_device, b.dtype, b.err, b.mode == FO_STATE_Q8,
+  const int rc = adam ? g_api.adam_step(segs, chunks, n, total, on_device(b), b.dtype, b.err, b.mode == FO_STATE_Q8,
                                         &ah, stream)
-                      : g_api.momentum_step(segs, chunks, n, total, on_device, b.dtype, b.err, b.mode, &mh, stream);
+                      : g_api.momentum_step(segs, chunks, n, total, on_device(b), b.dtype, b.err, b.mode, &mh, stream);
   if (g_nvtx) nvtxRangePop();
   return rc;
 }
@@ -380,6 +382,13 @@ bool ensure_status(c10::DeviceIndex device) {
   if (device < 64) g_status_ready |= uint64_t(1) << device;
   return true;
 }
+
+// Gives the GIL away for a scope.  What throws inside takes it back on its way out, before a
+// handler touches the interpreter.
+struct GilReleased {
+  PyThreadState* state = PyEval_SaveThread();
+  ~GilReleased() { PyEval_RestoreThread(state); }
+};
 
 struct Busy {
   bool& b;
@@ -451,6 +460,15 @@ PyObject* walker_step(Walker* w, PyObject* const* args, Py_ssize_t nargs) {
       if (c.adam && !adam_hyper(h, g.buckets[i]->step, ah[i])) Py_RETURN_FALSE;
     }
     if (!c.adam) momentum_hyper(h, mh);
+    for (size_t i = 0; i < g.used; ++i)
+      if (!ensure_status(g.buckets[i]->device)) return nullptr;
+    for (size_t i = 0; i < g.used; ++i) {
+      Bucket& b = *g.buckets[i];
+      if (!on_device(b)) continue;
+      GilReleased released;  // allocates and copies; whatever fails here leaves the step undone
+      c10::cuda::OptionalCUDAGuard guard(c10::Device(c10::DeviceType::CUDA, b.device));
+      upload(b);
+    }
 
     // from here on the call is committed
     for (PyObject* p : *w->skipped) {
@@ -463,13 +481,12 @@ PyObject* walker_step(Walker* w, PyObject* const* args, Py_ssize_t nargs) {
     }
     for (float* s : *w->steps) *s += 1.0f;
     for (size_t i = 0; i < g.used; ++i) {
-      Bucket& b = *g.buckets[i];
-      if (!ensure_status(b.device)) return nullptr;
-      int rc;
-      Py_BEGIN_ALLOW_THREADS
       static const FoAdamHyper none = {};
-      rc = launch(b, c.adam, c.adam ? ah[i] : none, mh);
-      Py_END_ALLOW_THREADS
+      int rc;
+      {
+        GilReleased released;
+        rc = launch(*g.buckets[i], c.adam, c.adam ? ah[i] : none, mh);
+      }
       if (rc) {
         PyErr_Format(g_native_error, "%s failed with CUDA error %d", c.adam ? "fo_adam_step" : "fo_momentum_step", rc);
         return nullptr;
@@ -481,8 +498,8 @@ PyObject* walker_step(Walker* w, PyObject* const* args, Py_ssize_t nargs) {
     if (!list) return nullptr;
     for (size_t i = 0; i < w->updated->size(); ++i) PyList_SET_ITEM(list, i, Py_NewRef((*w->updated)[i]));
     return list;
-  } catch (const std::exception& e) {
-    if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, e.what());
+  } catch (...) {  // as the Python exception that torch makes of it, OutOfMemoryError among them
+    if (!PyErr_Occurred()) torch::translate_exception_to_python(std::current_exception());
     return nullptr;
   }
 }

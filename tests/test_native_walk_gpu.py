@@ -113,3 +113,34 @@ def test_hooks_and_profiler_still_see_the_step():
     sched = torch.optim.lr_scheduler.StepLR(opt, 1)
     opt.step()
     sched.step()
+
+
+def test_an_allocation_that_fails_in_a_step_is_an_exception_and_leaves_the_step_undone():
+    """The address table of a long list does not fit any more: out of memory, raised as such, with
+    parameters, states and step counts as they were; the next step is made as if nothing had been."""
+    results = []
+    for short_of_memory in (True, False):
+        params, opt = _make(fo.FlashAdamW, {}, (torch.bfloat16,), 44)
+        _grads(params, 1, ())
+        opt.step()
+        _grads(params, 2, (4, 5))  # another number of rows, at other addresses
+        if short_of_memory:
+            before = _state_tensors(opt)
+            fill = []
+            torch.cuda.synchronize()
+            torch.cuda.empty_cache()
+            torch.cuda.set_per_process_memory_fraction(0.0)
+            try:
+                with pytest.raises(torch.OutOfMemoryError):
+                    while True:  # what is left in the allocator's small blocks
+                        fill.append(torch.empty(512, dtype=torch.uint8, device="cuda"))
+                with pytest.raises(torch.OutOfMemoryError):
+                    opt.step()
+            finally:
+                torch.cuda.set_per_process_memory_fraction(1.0)
+            for (_, a), (_, b) in zip(before, _state_tensors(opt)):
+                assert torch.equal(a, b)
+        opt.step()
+        results.append(_state_tensors(opt))
+    for (ka, a), (kb, b) in zip(*results):
+        assert ka == kb and torch.equal(a, b), ka
