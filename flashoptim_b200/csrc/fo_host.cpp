@@ -65,20 +65,32 @@ PyObject* slot(PyObject* o, Py_ssize_t off) {  // borrowed; null for None or nev
 }
 
 // ---------------------------------------------------------------- one launch
+// Device copy of a table that does not fit the kernel parameters.  It is written and read on one
+// stream, the one it was allocated on, and is not freed while its optimizer lives.
+struct Table {
+  c10::DeviceIndex device;
+  c10::StreamId stream;
+  int dtype, err, mode;
+  std::vector<FoSeg> sent;  // what `dev` holds; empty when that is not known
+  size_t n;                 // rows that it has room for, exactly
+  at::Tensor dev;
+  long long call = 0;       // last call that used it
+};
+
 struct Bucket {
   c10::DeviceIndex device;
   int dtype, err, mode;
   long long step;  // Adam only: bias corrections are per step count
   std::vector<FoSeg> rows;
   std::vector<int32_t> chunks;
-  // device copy of a table that does not fit the kernel parameters
-  std::vector<FoSeg> sent;
-  at::Tensor dev;
+  Table* table;
 };
 
 struct Group {
   std::vector<std::unique_ptr<Bucket>> buckets;
   size_t used = 0;
+  std::vector<std::unique_ptr<Table>> tables;
+  long long calls = 0;
 };
 
 struct Walker {
@@ -135,10 +147,6 @@ Bucket& bucket_for(Group& g, c10::DeviceIndex device, int dtype, int err, int mo
   }
   if (g.used == g.buckets.size()) g.buckets.push_back(std::make_unique<Bucket>());
   Bucket& b = *g.buckets[g.used++];
-  if (b.dev.defined() && b.dev.device().index() != device) {
-    b.dev = at::Tensor();
-    b.sent.clear();
-  }
   b.device = device;
   b.dtype = dtype;
   b.err = err;
@@ -333,20 +341,42 @@ bool prefix(Bucket& b) {
   return true;
 }
 
-// Device copy of a long table, re-sent only when a row changed (in steady state the caching
-// allocator returns gradients at the same addresses step after step).
-void upload(Bucket& b) {
+// The device copy of a long table, re-sent only when a row changed (in steady state the caching
+// allocator returns gradients at the same addresses step after step).  Each stream and number of
+// rows has a copy of its own, so that none is replaced when parameters come and go or written while
+// a launch on another stream reads it; two buckets of one call share none.
+void upload(Group& g, Bucket& b) {
   const size_t n = b.rows.size(), seg_bytes = n * sizeof(FoSeg), bytes = seg_bytes + (n + 1) * sizeof(int32_t);
-  if (b.dev.defined() && b.sent.size() == n && std::memcmp(b.sent.data(), b.rows.data(), seg_bytes) == 0) return;
-  b.sent.clear();  // any line below may throw; what the buffer holds is known again once all have passed
+  const c10::StreamId stream = c10::cuda::getCurrentCUDAStream(b.device).id();
+  Table* t = nullptr;
+  for (auto& have : g.tables)
+    if (have->n == n && have->call != g.calls && have->device == b.device && have->stream == stream &&
+        have->dtype == b.dtype && have->err == b.err && have->mode == b.mode) {
+      t = have.get();
+      break;
+    }
+  if (!t) {
+    auto fresh = std::make_unique<Table>();
+    fresh->device = b.device;
+    fresh->stream = stream;
+    fresh->dtype = b.dtype;
+    fresh->err = b.err;
+    fresh->mode = b.mode;
+    fresh->n = n;
+    fresh->dev = at::empty({(int64_t)bytes}, at::TensorOptions().dtype(at::kByte).device(
+                                                 c10::Device(c10::DeviceType::CUDA, b.device)));
+    t = fresh.get();
+    g.tables.push_back(std::move(fresh));
+  }
+  t->call = g.calls;
+  b.table = t;
+  if (t->sent.size() == n && std::memcmp(t->sent.data(), b.rows.data(), seg_bytes) == 0) return;
+  t->sent.clear();  // any line below may throw; what the buffer holds is known again once all have passed
   at::Tensor staged = at::empty({(int64_t)bytes}, at::TensorOptions().dtype(at::kByte).pinned_memory(true));
   std::memcpy(staged.data_ptr(), b.rows.data(), seg_bytes);
   std::memcpy(static_cast<char*>(staged.data_ptr()) + seg_bytes, b.chunks.data(), (n + 1) * sizeof(int32_t));
-  if (!b.dev.defined() || (size_t)b.dev.numel() != bytes)
-    b.dev = at::empty({(int64_t)bytes},
-                      at::TensorOptions().dtype(at::kByte).device(c10::Device(c10::DeviceType::CUDA, b.device)));
-  b.dev.copy_(staged, /*non_blocking=*/true);  // the host allocator keeps `staged` until the copy is done
-  b.sent = b.rows;
+  t->dev.copy_(staged, /*non_blocking=*/true);  // the host allocator keeps `staged` until the copy is done
+  t->sent = b.rows;
 }
 
 bool on_device(const Bucket& b) { return b.rows.size() > FO_MAX_INLINE_SEGS; }
@@ -358,7 +388,7 @@ int launch(Bucket& b, bool adam, const FoAdamHyper& ah, const FoMomentumHyper& m
   const FoSeg* segs = b.rows.data();
   const int32_t* chunks = b.chunks.data();
   if (on_device(b)) {
-    segs = static_cast<const FoSeg*>(b.dev.data_ptr());
+    segs = static_cast<const FoSeg*>(b.table->dev.data_ptr());
     chunks = reinterpret_cast<const int32_t*>(segs + n);
   }
   void* stream = c10::cuda::getCurrentCUDAStream(b.device).stream();
@@ -445,6 +475,7 @@ PyObject* walker_step(Walker* w, PyObject* const* args, Py_ssize_t nargs) {
     if (w->groups->size() <= slot_index) w->groups->resize(slot_index + 1);
     Group& g = (*w->groups)[slot_index];
     g.used = 0;
+    ++g.calls;
     w->steps->clear();
     w->updated->clear();
     w->skipped->clear();
@@ -467,7 +498,7 @@ PyObject* walker_step(Walker* w, PyObject* const* args, Py_ssize_t nargs) {
       if (!on_device(b)) continue;
       GilReleased released;  // allocates and copies; whatever fails here leaves the step undone
       c10::cuda::OptionalCUDAGuard guard(c10::Device(c10::DeviceType::CUDA, b.device));
-      upload(b);
+      upload(g, b);
     }
 
     // from here on the call is committed
@@ -514,6 +545,19 @@ PyObject* walker_new(PyTypeObject* type, PyObject*, PyObject*) {
   w->busy = false;
   return reinterpret_cast<PyObject*>(w);
 }
+// The device tables: a list of (rows, address).
+PyObject* walker_tables(Walker* w, PyObject*) {
+  PyObject* list = PyList_New(0);
+  if (w->busy) return list;  // another thread is writing them
+  for (size_t i = 0; list && i < w->groups->size(); ++i)
+    for (auto& t : (*w->groups)[i].tables) {
+      PyObject* item = Py_BuildValue("nn", (Py_ssize_t)t->n, (Py_ssize_t)t->dev.data_ptr());
+      if (!item || PyList_Append(list, item) < 0) Py_CLEAR(list);
+      Py_XDECREF(item);
+      if (!list) break;
+    }
+  return list;
+}
 void walker_dealloc(Walker* w) {
   delete w->groups;
   delete w->steps;
@@ -524,6 +568,7 @@ void walker_dealloc(Walker* w) {
 
 PyMethodDef walker_methods[] = {
     {"step", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(walker_step)), METH_FASTCALL, nullptr},
+    {"tables", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(walker_tables)), METH_NOARGS, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };
 

@@ -144,3 +144,33 @@ def test_an_allocation_that_fails_in_a_step_is_an_exception_and_leaves_the_step_
         results.append(_state_tensors(opt))
     for (ka, a), (kb, b) in zip(*results):
         assert ka == kb and torch.equal(a, b), ka
+
+
+def test_address_tables_are_not_freed_or_shared_under_a_launch_on_another_stream():
+    """Parameters come and go while steps run on two streams: every stream and number of rows keeps
+    its own table, and what the steps leave is what they leave on one stream."""
+    results = []
+    for streams in (2, 1):
+        params = [nn.Parameter(torch.linspace(-1, 1, 700 + i, device="cuda").bfloat16()) for i in range(40)]
+        opt = fo.FlashLion(params, lr=0.01)
+        other = torch.cuda.Stream() if streams == 2 else torch.cuda.current_stream()
+        seen = []
+        for it, (count, stream) in enumerate([(20, None), (20, other), (24, other), (20, other), (24, None), (40, other)]):
+            _grads(params, it, range(count, 40))
+            side = stream if stream is not None else torch.cuda.current_stream()
+            side.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(side):
+                torch.cuda._sleep(2_000_000)  # about a millisecond: the launches behind it are still to come
+                opt.step()
+            seen.append(dict.fromkeys(opt._walker.tables()))
+            assert all(t in seen[-1] for before in seen for t in before)
+            # nothing of a table's size that is allocated now lies where a table does
+            blocks = [torch.empty(n * 68 + 4, dtype=torch.uint8, device="cuda") for n in (20, 24) * 4]
+            assert not {b.data_ptr() for b in blocks} & {address for _, address in seen[-1]}
+            torch.cuda.current_stream().wait_stream(side)
+        torch.cuda.synchronize()
+        if streams == 2:
+            assert sorted(n for n, _ in seen[-1]) == [20, 20, 24, 24, 40]
+        results.append(_state_tensors(opt))
+    for (ka, a), (kb, b) in zip(*results):
+        assert ka == kb and torch.equal(a, b), ka
