@@ -17,6 +17,7 @@
 
 #include <ATen/ATen.h>
 #include <ATen/record_function.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <nvtx3/nvToolsExt.h>
@@ -74,6 +75,7 @@ struct Table {
   std::vector<FoSeg> sent;  // what `dev` holds; empty when that is not known
   size_t n;                 // rows that it has room for, exactly
   at::Tensor dev;
+  at::Tensor staged;        // of a captured step: its replays copy from here again
   long long call = 0;       // last call that used it
 };
 
@@ -344,13 +346,16 @@ bool prefix(Bucket& b) {
 // The device copy of a long table, re-sent only when a row changed (in steady state the caching
 // allocator returns gradients at the same addresses step after step).  Each stream and number of
 // rows has a copy of its own, so that none is replaced when parameters come and go or written while
-// a launch on another stream reads it; two buckets of one call share none.
+// a launch on another stream reads it; two buckets of one call share none.  A captured step gets
+// one that no other step shares: the copy runs when the graph is replayed, so that the host does
+// not know what the buffer holds, and what it copies from has to stay as long as the graph may.
 void upload(Group& g, Bucket& b) {
   const size_t n = b.rows.size(), seg_bytes = n * sizeof(FoSeg), bytes = seg_bytes + (n + 1) * sizeof(int32_t);
   const c10::StreamId stream = c10::cuda::getCurrentCUDAStream(b.device).id();
+  const bool capturing = c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;
   Table* t = nullptr;
   for (auto& have : g.tables)
-    if (have->n == n && have->call != g.calls && have->device == b.device && have->stream == stream &&
+    if (!capturing && !have->staged.defined() && have->n == n && have->call != g.calls && have->device == b.device && have->stream == stream &&
         have->dtype == b.dtype && have->err == b.err && have->mode == b.mode) {
       t = have.get();
       break;
@@ -375,6 +380,7 @@ void upload(Group& g, Bucket& b) {
   at::Tensor staged = at::empty({(int64_t)bytes}, at::TensorOptions().dtype(at::kByte).pinned_memory(true));
   std::memcpy(staged.data_ptr(), b.rows.data(), seg_bytes);
   std::memcpy(static_cast<char*>(staged.data_ptr()) + seg_bytes, b.chunks.data(), (n + 1) * sizeof(int32_t));
+  if (capturing) t->staged = staged;
   t->dev.copy_(staged, /*non_blocking=*/true);  // the host allocator keeps `staged` until the copy is done
   t->sent = b.rows;
 }
@@ -545,13 +551,14 @@ PyObject* walker_new(PyTypeObject* type, PyObject*, PyObject*) {
   w->busy = false;
   return reinterpret_cast<PyObject*>(w);
 }
-// The device tables: a list of (rows, address).
+// The device tables: a list of (rows, address, host address that replays copy from or 0).
 PyObject* walker_tables(Walker* w, PyObject*) {
   PyObject* list = PyList_New(0);
   if (w->busy) return list;  // another thread is writing them
   for (size_t i = 0; list && i < w->groups->size(); ++i)
     for (auto& t : (*w->groups)[i].tables) {
-      PyObject* item = Py_BuildValue("nn", (Py_ssize_t)t->n, (Py_ssize_t)t->dev.data_ptr());
+      PyObject* item = Py_BuildValue("nnn", (Py_ssize_t)t->n, (Py_ssize_t)t->dev.data_ptr(),
+                                     t->staged.defined() ? (Py_ssize_t)t->staged.data_ptr() : (Py_ssize_t)0);
       if (!item || PyList_Append(list, item) < 0) Py_CLEAR(list);
       Py_XDECREF(item);
       if (!list) break;

@@ -170,6 +170,8 @@ class SegmentTable:
         self._chunks: Optional[np.ndarray] = None     # [n_seg + 1] int32
         self._dev: Optional[torch.Tensor] = None      # uint8 device buffer: segs then chunk_begin
         self._chunk = 0                               # chunk size the prefix was built for
+        # (host, device) image of every captured launch: a replay copies from the one to the other
+        self._captured: list[tuple[torch.Tensor, torch.Tensor]] = []
         self.uploads = 0
 
     @staticmethod
@@ -202,18 +204,26 @@ class SegmentTable:
         if n_seg <= native.FO_MAX_INLINE_SEGS and not force_device:
             self._host = rows
             return rows.ctypes.data, self._chunks.ctypes.data, n_seg, total, 0
-        if changed or self._dev is None:
+        # a captured copy runs when the graph is replayed: it has images of its own, both kept
+        capturing = torch.cuda.is_current_stream_capturing()
+        dev = None if capturing else self._dev
+        if changed or dev is None:
             seg_bytes = n_seg * SEG_WORDS * 8
             img = np.empty(seg_bytes + (n_seg + 1) * 4, dtype=np.uint8)
             img[:seg_bytes] = rows.reshape(-1).view(np.uint8)
             img[seg_bytes:] = self._chunks.view(np.uint8)
             staged = torch.from_numpy(img).pin_memory()
-            if self._dev is None or self._dev.numel() != img.size:
-                self._dev = torch.empty(img.size, dtype=torch.uint8, device=self.device)
-            self._dev.copy_(staged, non_blocking=True)
-            self._host = rows.copy()
+            if dev is None or dev.numel() != img.size:
+                dev = torch.empty(img.size, dtype=torch.uint8, device=self.device)
+            dev.copy_(staged, non_blocking=True)
             self.uploads += 1
-        base = self._dev.data_ptr()
+            if capturing:
+                self._captured.append((staged, dev))
+                self._host = None  # the prefix in hand is this launch's
+            else:
+                self._dev = dev
+                self._host = rows.copy()
+        base = dev.data_ptr()
         return base, base + n_seg * SEG_WORDS * 8, n_seg, total, 1
 
 

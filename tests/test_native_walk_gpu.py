@@ -166,11 +166,66 @@ def test_address_tables_are_not_freed_or_shared_under_a_launch_on_another_stream
             assert all(t in seen[-1] for before in seen for t in before)
             # nothing of a table's size that is allocated now lies where a table does
             blocks = [torch.empty(n * 68 + 4, dtype=torch.uint8, device="cuda") for n in (20, 24) * 4]
-            assert not {b.data_ptr() for b in blocks} & {address for _, address in seen[-1]}
+            assert not {b.data_ptr() for b in blocks} & {t[1] for t in seen[-1]}
             torch.cuda.current_stream().wait_stream(side)
         torch.cuda.synchronize()
         if streams == 2:
-            assert sorted(n for n, _ in seen[-1]) == [20, 20, 24, 24, 40]
+            assert sorted(t[0] for t in seen[-1]) == [20, 20, 24, 24, 40]
+        results.append(_state_tensors(opt))
+    for (ka, a), (kb, b) in zip(*results):
+        assert ka == kb and torch.equal(a, b), ka
+
+
+@pytest.mark.parametrize("native", [True, False])
+def test_a_captured_step_keeps_its_address_table(native, monkeypatch):
+    """Steps between capture and replay, on other gradients and with another number of rows, change
+    nothing about what a replay updates from, and a replay nothing about what the next step does."""
+    results = []
+    for capture in (True, False):
+        params = [nn.Parameter(torch.linspace(-1, 1, 700 + i, device="cuda").bfloat16()) for i in range(30)]
+        opt = fo.FlashLion(params, lr=0.01)
+        if not native:
+            monkeypatch.setattr(opt, "_native_step_group", lambda *a: False)
+
+        def step(seed, count):
+            _grads(params, seed, range(count, 30))
+            opt.step()
+
+        step(0, 20)
+        _grads(params, 1, range(20, 30))
+        held = [p.grad for p in params]  # the captured step's gradients
+        if capture:
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                opt.step()
+                opt.step()
+
+        def replay():
+            if capture:
+                graph.replay()
+                return
+            now = [p.grad for p in params]
+            for again in (0, 1):
+                for p, g in zip(params, held):
+                    p.grad = g
+                opt.step()
+            for p, g in zip(params, now):
+                p.grad = g
+
+        opt.step()  # the rows of the captured step, before its copies have run once
+        step(2, 24)
+        if capture and native:
+            kept = {t[2] for t in opt._walker.tables()} - {0}
+            assert len(kept) == 2
+            blocks = [torch.empty(20 * 68 + 4, dtype=torch.uint8).pin_memory() for _ in range(8)]
+            assert not {b.data_ptr() for b in blocks} & kept
+        replay()
+        step(3, 20)
+        replay()
+        opt.step()
+        replay()
+        replay()
+        torch.cuda.synchronize()
         results.append(_state_tensors(opt))
     for (ka, a), (kb, b) in zip(*results):
         assert ka == kb and torch.equal(a, b), ka
