@@ -49,6 +49,10 @@ from .state import MaybeQuantizedTensor, QuantizedTensorSpec
 _torch_optimizer = importlib.import_module(torch.optim.Optimizer.__module__)
 _global_step_hooks = [getattr(_torch_optimizer, f"_global_optimizer_{when}_hooks", (None,)) for when in ("pre", "post")]
 
+# What the native walk does in place of these methods is what they do in the class that says so
+# (_native_step_args); where one of them was overridden since, the Python walk calls it.
+_WALKED = ("_pre_step", "_pre_step_many", "_fused_step", "_step_group", "_ensure_state_initialized")
+
 _VALID_MASTER_WEIGHT_BITS = (None, 24, 32)
 _BITS_TO_BYTES = {None: 0, 24: 3, 32: 4}
 
@@ -106,6 +110,13 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
             every parameter is fp32 (no effect; override with the environment
             variable ``FLASHOPTIM_ALLOW_INEFFECTIVE_MASTER_WEIGHT_BITS``).
     """
+
+    _walked_natively: tuple = ()  # the methods that the native walk stands for
+
+    def __init_subclass__(cls, **kwargs: Any) -> None:
+        super().__init_subclass__(**kwargs)
+        if "_native_step_args" in cls.__dict__:
+            cls._walked_natively = tuple(getattr(cls, name) for name in _WALKED)
 
     def __init__(
         self,
@@ -231,7 +242,8 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
     def _native_step_args(self, hparams: dict[str, Any]) -> Optional[tuple[tuple[str, ...], bool, tuple]]:
         """What the native walk needs to know about a group: names of the moments in kernel
         order, whether the rule is Adam's, and its scalars (``csrc/fo_host.cpp``, ``adam_hyper``
-        and ``momentum_hyper``).  None: this class is stepped by the Python walk only."""
+        and ``momentum_hyper``).  None: this class is stepped by the Python walk only, as is one
+        that overrides a method of ``_WALKED`` below the class that defines this one."""
         return None
 
     def _initial_value_for_state_var(self, param: torch.Tensor, key: str) -> torch.Tensor:
@@ -368,9 +380,18 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
                 return i
         return -1
 
+    def _overrides_the_walk(self) -> bool:
+        cls, own = type(self), self.__dict__  # of the class, or of the instance; written out, as every step asks
+        return (
+            (cls._pre_step, cls._pre_step_many, cls._fused_step, cls._step_group, cls._ensure_state_initialized)
+            != cls._walked_natively
+            or "_pre_step" in own or "_pre_step_many" in own or "_fused_step" in own or "_step_group" in own
+            or "_ensure_state_initialized" in own
+        )
+
     def _native_step_group(self, params: list[torch.Tensor], group: dict[str, Any], group_index: int) -> bool:
         """:meth:`_step_group` in native code.  False: nothing was changed, walk in Python."""
-        if not self._fused or not params or not params[0].is_cuda:
+        if not self._fused or not params or not params[0].is_cuda or self._overrides_the_walk():
             return False
         args = self._native_step_args(group)
         if args is None:

@@ -1,0 +1,71 @@
+"""Which steps the native walk may take: what a subclass, a patch or an instance overrides is called."""
+
+import pytest
+import torch
+import torch.nn as nn
+
+import flashoptim_b200 as fo
+
+OVERRIDES = ["_pre_step", "_pre_step_many", "_fused_step", "_step_group", "_ensure_state_initialized"]
+CLASSES = [fo.FlashAdam, fo.FlashAdamW, fo.FlashLion, fo.FlashSGD, fo.FlashSGDW]
+
+
+def _param(device="cpu"):
+    return nn.Parameter(torch.ones(100, device=device).bfloat16())
+
+
+def _counting(cls, name, calls):
+    def method(self, *args, **kwargs):
+        calls.append(name)
+        return getattr(super(sub, self), name)(*args, **kwargs)
+
+    sub = type("Sub", (cls,), {name: method})
+    return sub
+
+
+@pytest.mark.parametrize("cls", CLASSES)
+@pytest.mark.parametrize("name", OVERRIDES)
+def test_an_override_keeps_the_native_walk_out(cls, name, monkeypatch):
+    assert not cls([_param()], lr=0.1)._overrides_the_walk()
+    assert not type("Plain", (cls,), {})([_param()], lr=0.1)._overrides_the_walk()
+    sub = _counting(cls, name, [])
+    assert sub([_param()], lr=0.1)._overrides_the_walk()
+    assert type("SubSub", (sub,), {})([_param()], lr=0.1)._overrides_the_walk()
+    opt = cls([_param()], lr=0.1)
+    setattr(opt, name, getattr(opt, name))
+    assert opt._overrides_the_walk()
+    opt = cls([_param()], lr=0.1)
+    original = getattr(cls, name)
+    monkeypatch.setattr(cls, name, lambda *a, **k: original(*a, **k))
+    assert opt._overrides_the_walk()
+
+
+def test_a_class_that_says_what_it_does_is_walked_natively():
+    class Own(fo.FlashLion):
+        def _pre_step_many(self, param_states):
+            pass
+
+        def _native_step_args(self, hparams):
+            return super()._native_step_args(hparams)
+
+    assert not Own([_param()], lr=0.1)._overrides_the_walk()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cls", [fo.FlashAdamW, fo.FlashLion, fo.FlashSGDW])
+@pytest.mark.parametrize("name", OVERRIDES)
+def test_an_override_is_called_on_the_gpu_as_on_the_cpu(cls, name):
+    calls = {"cpu": [], "cuda": []}
+    for device, seen in calls.items():
+        p = _param(device)
+        opt = _counting(cls, name, seen)([p], lr=0.1)
+        for _ in range(2):
+            p.grad = torch.ones_like(p)
+            opt.step()
+            opt.step_param(p)
+    if name == "_pre_step" and cls is fo.FlashAdamW:
+        return  # Adam counts the steps of a fused launch in _pre_step_many; _pre_step is the eager path's
+    if name in ("_pre_step_many", "_fused_step"):
+        assert len(calls["cuda"]) == 4 and not calls["cpu"]
+    else:
+        assert len(calls["cuda"]) == len(calls["cpu"]) == 4
