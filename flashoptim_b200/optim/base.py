@@ -31,6 +31,7 @@ What differs by design:
 from __future__ import annotations
 
 import abc
+import functools
 import importlib
 import math
 import os
@@ -47,7 +48,8 @@ from .state import MaybeQuantizedTensor, QuantizedTensorSpec
 
 # Step hooks that apply to every optimizer of the process; where torch does not show them, assume some.
 _torch_optimizer = importlib.import_module(torch.optim.Optimizer.__module__)
-_global_step_hooks = [getattr(_torch_optimizer, f"_global_optimizer_{when}_hooks", (None,)) for when in ("pre", "post")]
+_global_pre_hooks = getattr(_torch_optimizer, "_global_optimizer_pre_hooks", (None,))
+_global_post_hooks = getattr(_torch_optimizer, "_global_optimizer_post_hooks", (None,))
 
 # What the native walk does in place of these methods is what they do in the class that says so
 # (_native_step_args); where one of them was overridden since, the Python walk calls it.
@@ -472,23 +474,24 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
         if not self._native_step_group([p], group, index):
             self._step_group([p], group, index)
 
+    @staticmethod
+    def profile_hook_step(func: Callable) -> Callable:
+        """What torch wraps the ``step()`` of a class in, when the first instance is made: a profiler
+        annotation and the step hooks.  They cost 9 us of a call that otherwise takes about as long,
+        so they are passed by while nobody profiles and no hook is registered."""
+        observed = torch.optim.Optimizer.profile_hook_step(func)
+
+        @functools.wraps(func)
+        def step(self, *args, **kwargs):
+            mod = host.loaded()
+            if (mod is None or mod.observed() or self._optimizer_step_pre_hooks or self._optimizer_step_post_hooks
+                    or _global_pre_hooks or _global_post_hooks):
+                return observed(self, *args, **kwargs)
+            return func(self, *args, **kwargs)
+
+        return step
+
     def step(self, closure: Optional[Callable] = None) -> Optional[torch.Tensor]:
-        # torch wraps the step() of every optimizer class in a profiler annotation and its step
-        # hooks, which costs 9 us of a call that otherwise takes about as long.  This one (marked
-        # as wrapped already, below) takes that route only when somebody profiles or has
-        # registered a hook; a subclass with a step() of its own is wrapped by torch as usual.
-        mod = host.loaded()
-        if type(self).step is not FlashOptimizer.step or (
-            mod is not None and not mod.observed()
-            and not self._optimizer_step_pre_hooks and not self._optimizer_step_post_hooks
-            and not any(_global_step_hooks)
-        ):
-            return self._step(closure)
-        return _observed_step(self, closure)
-
-    step.hooked = True
-
-    def _step(self, closure: Optional[Callable] = None) -> Optional[torch.Tensor]:
         if self._gradient_release:
             warnings.warn(
                 "gradient release is active: the gradient hooks already update the parameters during "
@@ -814,7 +817,3 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
             if "error_bits" in state:
                 width = local_param.element_size() + state["error_bits"].element_size()
                 state["error_bits"] = compute_ecc_bits(local_value, local_param, master_bytewidth=width)
-
-
-# step() with torch's profiler annotation and step hooks around it
-_observed_step = torch.optim.Optimizer.profile_hook_step(FlashOptimizer._step)
