@@ -44,7 +44,7 @@ bool g_nvtx = false;
 uint64_t g_status_ready = 0;  // bit per device whose kernels know their status word
 long long g_launches = 0;
 
-PyObject *s_step, *s_error_bits, *s_local_tensor, *s_ensure, *s_check;
+PyObject *s_step, *s_error_bits, *s_local_tensor, *s_ensure, *s_check, *s_walked_natively;
 
 // Slots of MaybeQuantizedTensor, read at their offsets: an attribute look-up per slot would be a
 // quarter of the whole walk.
@@ -63,6 +63,30 @@ Py_ssize_t slot_offset(PyTypeObject* type, const char* name) {
 PyObject* slot(PyObject* o, Py_ssize_t off) {  // borrowed; null for None or never assigned
   PyObject* v = *reinterpret_cast<PyObject**>(reinterpret_cast<char*>(o) + off);
   return v == Py_None ? nullptr : v;
+}
+
+// The methods whose place the walk takes, by name.  A class that describes its rule to the walk
+// keeps those that it describes in `_walked_natively` (optim/base.py).
+PyObject* g_walked = nullptr;
+
+// Whether the class of `opt`, or `opt` itself, has other methods than those; -1 with an exception.
+int overrides(PyObject* opt) {
+  PyObject* type = reinterpret_cast<PyObject*>(Py_TYPE(opt));
+  PyObject* known = PyObject_GetAttr(type, s_walked_natively);
+  if (!known) return -1;
+  PyObject* own = PyObject_GenericGetDict(opt, nullptr);
+  const Py_ssize_t n = PyTuple_GET_SIZE(g_walked);
+  int other = own ? !PyTuple_Check(known) || PyTuple_GET_SIZE(known) != n : -1;
+  for (Py_ssize_t i = 0; !other && i < n; ++i) {
+    PyObject* name = PyTuple_GET_ITEM(g_walked, i);
+    PyObject* now = PyObject_GetAttr(type, name);
+    other = now ? now != PyTuple_GET_ITEM(known, i) : -1;
+    Py_XDECREF(now);
+    if (!other) other = PyDict_Contains(own, name);
+  }
+  Py_XDECREF(own);
+  Py_DECREF(known);
+  return other;
 }
 
 // ---------------------------------------------------------------- one launch
@@ -432,6 +456,7 @@ struct Busy {
   ~Busy() { b = false; }
 };
 
+// Nothing is done for an optimizer with methods of its own in the walk's place.
 // Walker.step(opt, params, state, ready, skip, group, group_index, keys, adam, check, listeners,
 //             hyper) -> False (nothing done, not served), True, or the list of updated parameters.
 PyObject* walker_step(Walker* w, PyObject* const* args, Py_ssize_t nargs) {
@@ -440,6 +465,10 @@ PyObject* walker_step(Walker* w, PyObject* const* args, Py_ssize_t nargs) {
     return nullptr;
   }
   if (w->busy) Py_RETURN_FALSE;  // another thread is inside a launch of this optimizer
+  if (const int other = overrides(args[0])) {
+    if (other < 0) return nullptr;
+    Py_RETURN_FALSE;
+  }
   Call c;
   c.opt = args[0];
   c.params = args[1];
@@ -591,12 +620,13 @@ PyTypeObject walker_type = [] {
 }();
 
 // ---------------------------------------------------------------- module
-// setup(adam_step, momentum_step, chunk, state_type, ensure_status, native_error, nvtx)
+// setup(adam_step, momentum_step, chunk, state_type, ensure_status, native_error, nvtx, walked)
 PyObject* host_setup(PyObject*, PyObject* args) {
   unsigned long long adam, mom;
   int chunk, nvtx;
-  PyObject *type, *ensure, *error;
-  if (!PyArg_ParseTuple(args, "KKiO!OOp", &adam, &mom, &chunk, &PyType_Type, &type, &ensure, &error, &nvtx))
+  PyObject *type, *ensure, *error, *walked;
+  if (!PyArg_ParseTuple(args, "KKiO!OOpO!", &adam, &mom, &chunk, &PyType_Type, &type, &ensure, &error, &nvtx,
+                        &PyTuple_Type, &walked))
     return nullptr;
   PyTypeObject* t = reinterpret_cast<PyTypeObject*>(type);
   g_off_data = slot_offset(t, "_data");
@@ -609,6 +639,7 @@ PyObject* host_setup(PyObject*, PyObject* args) {
   g_nvtx = nvtx != 0;
   Py_XSETREF(g_ensure_status, Py_NewRef(ensure));
   Py_XSETREF(g_native_error, Py_NewRef(error));
+  Py_XSETREF(g_walked, Py_NewRef(walked));
   PyTypeObject* old = g_state_type;
   g_state_type = reinterpret_cast<PyTypeObject*>(Py_NewRef(type));
   Py_XDECREF(old);
@@ -616,6 +647,11 @@ PyObject* host_setup(PyObject*, PyObject* args) {
 }
 
 PyObject* host_launches(PyObject*, PyObject*) { return PyLong_FromLongLong(g_launches); }
+
+PyObject* host_overrides(PyObject*, PyObject* opt) {
+  const int other = overrides(opt);
+  return other < 0 ? nullptr : PyBool_FromLong(other);
+}
 
 // Whether somebody (a profiler, an execution trace) observes operator calls right now.
 PyObject* host_observed(PyObject*, PyObject*) {
@@ -625,6 +661,7 @@ PyObject* host_observed(PyObject*, PyObject*) {
 PyMethodDef host_methods[] = {
     {"setup", host_setup, METH_VARARGS, nullptr},
     {"launches", host_launches, METH_NOARGS, nullptr},
+    {"overrides", host_overrides, METH_O, nullptr},
     {"observed", host_observed, METH_NOARGS, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };
@@ -638,7 +675,8 @@ PyMODINIT_FUNC PyInit__fo_host() {
   s_local_tensor = PyUnicode_InternFromString("_local_tensor");
   s_ensure = PyUnicode_InternFromString("_ensure_state_initialized");
   s_check = PyUnicode_InternFromString("_check_param_numerics");
-  if (!s_step || !s_error_bits || !s_local_tensor || !s_ensure || !s_check) return nullptr;
+  s_walked_natively = PyUnicode_InternFromString("_walked_natively");
+  if (!s_walked_natively || !s_step || !s_error_bits || !s_local_tensor || !s_ensure || !s_check) return nullptr;
   if (PyType_Ready(&walker_type) < 0) return nullptr;
   PyObject* m = PyModule_Create(&host_module);
   if (!m) return nullptr;

@@ -40,12 +40,13 @@ def load() -> ModuleType:
         spec = importlib.util.spec_from_file_location("_fo_host", str(_build.HOST_PATH), loader=loader)
         mod = importlib.util.module_from_spec(spec)
         loader.exec_module(mod)
+        from ..optim.base import WALKED
         from ..optim.state import MaybeQuantizedTensor
 
         def address(fn) -> int:
             return ctypes.cast(fn, ctypes.c_void_p).value
 
         mod.setup(address(lib.fo_adam_step), address(lib.fo_momentum_step), native.chunk_elems(),
-                  MaybeQuantizedTensor, step._ensure_status, native.NativeError, step._NVTX)
+                  MaybeQuantizedTensor, step._ensure_status, native.NativeError, step._NVTX, WALKED)
         _module = mod
     return mod

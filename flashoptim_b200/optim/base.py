@@ -52,8 +52,9 @@ _global_pre_hooks = getattr(_torch_optimizer, "_global_optimizer_pre_hooks", (No
 _global_post_hooks = getattr(_torch_optimizer, "_global_optimizer_post_hooks", (None,))
 
 # What the native walk does in place of these methods is what they do in the class that says so
-# (_native_step_args); where one of them was overridden since, the Python walk calls it.
-_WALKED = ("_pre_step", "_pre_step_many", "_fused_step", "_step_group", "_ensure_state_initialized")
+# (_native_step_args); where one of them was overridden since, in a class or on an instance, the
+# Python walk calls it (csrc/fo_host.cpp, overrides).
+WALKED = ("_pre_step", "_pre_step_many", "_fused_step", "_step_group", "_ensure_state_initialized")
 
 _VALID_MASTER_WEIGHT_BITS = (None, 24, 32)
 _BITS_TO_BYTES = {None: 0, 24: 3, 32: 4}
@@ -118,7 +119,7 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
     def __init_subclass__(cls, **kwargs: Any) -> None:
         super().__init_subclass__(**kwargs)
         if "_native_step_args" in cls.__dict__:
-            cls._walked_natively = tuple(getattr(cls, name) for name in _WALKED)
+            cls._walked_natively = tuple(getattr(cls, name) for name in WALKED)
 
     def __init__(
         self,
@@ -245,7 +246,7 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
         """What the native walk needs to know about a group: names of the moments in kernel
         order, whether the rule is Adam's, and its scalars (``csrc/fo_host.cpp``, ``adam_hyper``
         and ``momentum_hyper``).  None: this class is stepped by the Python walk only, as is one
-        that overrides a method of ``_WALKED`` below the class that defines this one."""
+        that overrides a method of ``WALKED`` below the class that defines this one."""
         return None
 
     def _initial_value_for_state_var(self, param: torch.Tensor, key: str) -> torch.Tensor:
@@ -382,18 +383,9 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
                 return i
         return -1
 
-    def _overrides_the_walk(self) -> bool:
-        cls, own = type(self), self.__dict__  # of the class, or of the instance; written out, as every step asks
-        return (
-            (cls._pre_step, cls._pre_step_many, cls._fused_step, cls._step_group, cls._ensure_state_initialized)
-            != cls._walked_natively
-            or "_pre_step" in own or "_pre_step_many" in own or "_fused_step" in own or "_step_group" in own
-            or "_ensure_state_initialized" in own
-        )
-
     def _native_step_group(self, params: list[torch.Tensor], group: dict[str, Any], group_index: int) -> bool:
         """:meth:`_step_group` in native code.  False: nothing was changed, walk in Python."""
-        if not self._fused or not params or not params[0].is_cuda or self._overrides_the_walk():
+        if not self._fused or not params or not params[0].is_cuda:
             return False
         args = self._native_step_args(group)
         if args is None:
@@ -487,7 +479,9 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
             if (mod is None or mod.observed() or self._optimizer_step_pre_hooks or self._optimizer_step_post_hooks
                     or _global_pre_hooks or _global_post_hooks):
                 return observed(self, *args, **kwargs)
-            return func(self, *args, **kwargs)
+            if args or kwargs:
+                return func(self, *args, **kwargs)
+            return func(self)
 
         return step
 

@@ -5,6 +5,7 @@ import torch
 import torch.nn as nn
 
 import flashoptim_b200 as fo
+from flashoptim_b200.ops import host
 
 OVERRIDES = ["_pre_step", "_pre_step_many", "_fused_step", "_step_group", "_ensure_state_initialized"]
 CLASSES = [fo.FlashAdam, fo.FlashAdamW, fo.FlashLion, fo.FlashSGD, fo.FlashSGDW]
@@ -26,18 +27,18 @@ def _counting(cls, name, calls):
 @pytest.mark.parametrize("cls", CLASSES)
 @pytest.mark.parametrize("name", OVERRIDES)
 def test_an_override_keeps_the_native_walk_out(cls, name, monkeypatch):
-    assert not cls([_param()], lr=0.1)._overrides_the_walk()
-    assert not type("Plain", (cls,), {})([_param()], lr=0.1)._overrides_the_walk()
+    assert not host.load().overrides(cls([_param()], lr=0.1))
+    assert not host.load().overrides(type("Plain", (cls,), {})([_param()], lr=0.1))
     sub = _counting(cls, name, [])
-    assert sub([_param()], lr=0.1)._overrides_the_walk()
-    assert type("SubSub", (sub,), {})([_param()], lr=0.1)._overrides_the_walk()
+    assert host.load().overrides(sub([_param()], lr=0.1))
+    assert host.load().overrides(type("SubSub", (sub,), {})([_param()], lr=0.1))
     opt = cls([_param()], lr=0.1)
     setattr(opt, name, getattr(opt, name))
-    assert opt._overrides_the_walk()
+    assert host.load().overrides(opt)
     opt = cls([_param()], lr=0.1)
     original = getattr(cls, name)
     monkeypatch.setattr(cls, name, lambda *a, **k: original(*a, **k))
-    assert opt._overrides_the_walk()
+    assert host.load().overrides(opt)
 
 
 def test_a_class_that_says_what_it_does_is_walked_natively():
@@ -48,7 +49,7 @@ def test_a_class_that_says_what_it_does_is_walked_natively():
         def _native_step_args(self, hparams):
             return super()._native_step_args(hparams)
 
-    assert not Own([_param()], lr=0.1)._overrides_the_walk()
+    assert not host.load().overrides(Own([_param()], lr=0.1))
 
 
 @pytest.mark.gpu
