@@ -391,7 +391,10 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
         if args is None:
             return False
         if self._walker is None:
-            self._walker = host.load().Walker()
+            mod = host.available()
+            if mod is None:
+                return False
+            self._walker = mod.Walker()
         keys, adam, scalars = args
         listeners = self._local_update_listeners
         done = self._walker.step(

@@ -5,7 +5,8 @@ import torch
 import torch.nn as nn
 
 import flashoptim_b200 as fo
-from flashoptim_b200.ops import host
+from flashoptim_b200 import build
+from flashoptim_b200.ops import host, native
 
 OVERRIDES = ["_pre_step", "_pre_step_many", "_fused_step", "_step_group", "_ensure_state_initialized"]
 CLASSES = [fo.FlashAdam, fo.FlashAdamW, fo.FlashLion, fo.FlashSGD, fo.FlashSGDW]
@@ -70,3 +71,54 @@ def test_an_override_is_called_on_the_gpu_as_on_the_cpu(cls, name):
         assert len(calls["cuda"]) == 4 and not calls["cpu"]
     else:
         assert len(calls["cuda"]) == len(calls["cpu"]) == 4
+
+
+def _no_extension(monkeypatch, tried):
+    def build_host(*args, **kwargs):
+        tried.append(1)
+        raise RuntimeError("no C++ compiler")
+
+    monkeypatch.setattr(host, "_module", None)
+    monkeypatch.setattr(host, "_unavailable", False)
+    monkeypatch.setattr(build, "host_is_current", lambda: False)
+    monkeypatch.setattr(build, "build_host", build_host)
+
+
+def test_an_extension_that_cannot_be_built_is_reported_once(monkeypatch):
+    tried = []
+    _no_extension(monkeypatch, tried)
+    monkeypatch.setattr(native, "load", lambda path=None: None)
+    with pytest.warns(UserWarning, match="no C\\+\\+ compiler"):
+        assert host.available() is None
+    assert host.available() is None and len(tried) == 1  # neither warned of nor tried again
+
+
+def test_kernels_that_cannot_be_loaded_are_an_error(monkeypatch):
+    def load(path=None):
+        raise native.NativeError("missing")
+
+    _no_extension(monkeypatch, [])
+    monkeypatch.setattr(native, "load", load)
+    with pytest.raises(native.NativeError, match="missing"):
+        host.available()
+
+
+@pytest.mark.gpu
+def test_steps_without_the_extension_are_the_same_steps(monkeypatch):
+    results = []
+    for extension in (True, False):
+        if not extension:
+            _no_extension(monkeypatch, [])
+        params = [nn.Parameter(torch.linspace(-1, 1, 700 + i, device="cuda").bfloat16()) for i in range(20)]
+        opt = fo.FlashAdamW(params, lr=0.1)
+        for p in params:
+            p.grad = torch.ones_like(p)
+        if extension:
+            opt.step()
+        else:
+            with pytest.warns(UserWarning, match="Python walk"):
+                opt.step()
+        opt.step_param(params[0])
+        assert extension == (opt._walker is not None)
+        results.append(torch.cat([p.detach() for p in params]))
+    assert torch.equal(*results)
