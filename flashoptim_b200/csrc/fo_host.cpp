@@ -16,6 +16,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <ATen/ATen.h>
+#include <ATen/core/grad_mode.h>
 #include <ATen/record_function.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -504,6 +505,7 @@ PyObject* walker_step(Walker* w, PyObject* const* args, Py_ssize_t nargs) {
   for (Py_ssize_t i = 0; i < n_flags; ++i) h.flag[i] = PyObject_IsTrue(PyTuple_GET_ITEM(args[11], n_vals + i));
 
   Busy busy(w->busy);
+  at::NoGradGuard no_grad;  // for the Python methods that the walk calls: state creation, numerics check
   try {
     // groups are numbered from -1 (a group dict that the optimizer does not own)
     const size_t slot_index = (size_t)(c.group_index + 1);

@@ -403,8 +403,9 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
         if done is False:
             return False
         if listeners and done:
-            for fn in listeners:
-                fn(done)
+            with torch.no_grad():
+                for fn in listeners:
+                    fn(done)
         return True
 
     @torch.no_grad()

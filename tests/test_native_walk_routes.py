@@ -122,3 +122,27 @@ def test_steps_without_the_extension_are_the_same_steps(monkeypatch):
         assert extension == (opt._walker is not None)
         results.append(torch.cat([p.detach() for p in params]))
     assert torch.equal(*results)
+
+
+@pytest.mark.parametrize("device", ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)])
+def test_what_a_step_calls_runs_without_gradients(device):
+    modes = {}
+
+    class Lion(fo.FlashLion):
+        def _initial_value_for_state_var(self, param, key):
+            modes["state"] = torch.is_grad_enabled()
+            return torch.zeros_like(param)
+
+        def _check_param_numerics(self, *args):
+            modes["check"] = torch.is_grad_enabled()
+
+    for how in ("step", "step_param"):
+        p = _param(device)
+        opt = Lion([p], lr=0.1, check_numerics=True)
+        opt._local_update_listeners.append(lambda params: modes.update(listener=torch.is_grad_enabled()))
+        opt._post_step_callbacks.append(lambda: modes.update(callback=torch.is_grad_enabled()))
+        p.grad = torch.ones_like(p)
+        modes.clear()
+        opt.step() if how == "step" else opt.step_param(p)
+        assert torch.is_grad_enabled() and not any(modes.values())
+        assert set(modes) == {"state", "check", "listener"} | ({"callback"} if how == "step" else set())
