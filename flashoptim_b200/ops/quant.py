@@ -33,15 +33,31 @@ def _splits(param: torch.Tensor, error_bits: torch.Tensor) -> bool:
 
 class Conversions:
     """Conversions of many CUDA tensors, gathered and launched together: one launch per kind and
-    12 tensors instead of one per tensor.  Inputs are kept alive until :meth:`launch`, which comes by
-    itself when they reach ``HELD`` bytes: they may be copies (of a checkpoint in host memory), of
-    which a loop over tensors would hold one at a time."""
+    12 tensors instead of one per tensor.  Inputs are kept alive until :meth:`launch`.  Those that
+    were made for the list (device copies of a checkpoint in host memory, conversions of layout or
+    dtype) would each be freed after their tensor by a loop: when they reach ``HELD`` bytes, the list
+    is launched.  Inputs that live anyway cut it at ``WORK`` bytes, so that the device does not wait
+    for the whole walk."""
 
-    HELD = 1 << 30  # at 256 MB, a load of 1.3 GB took 555 us instead of 429: its launches got too small
+    HELD = 32 << 20  # launching costs about 40 us of the host, copying as much from host memory milliseconds
+    # Loading 1.3 GB from the device, whose walk takes the host as long as the conversions take the
+    # device: 511 us a call among others and 696 alone; 471 and 773 uncut, 555 and 652 at 512 MB, 590
+    # and 657 at 256 MB.  Exporting and importing 436 M elements: within 3 % among others from 256 MB
+    # on, 630 and 660 alone, 560 and 590 at 256 MB.
+    WORK = 1 << 30
 
     def __init__(self) -> None:
         self._lists: dict[Any, tuple[list[int], list[Any]]] = {}
-        self._held = 0
+        self._copies: set[int] = set()  # addresses of inputs that were made for the list
+        self._held = self._work = 0
+
+    def adopt(self, t: torch.Tensor) -> torch.Tensor:
+        """``t``, an input that was made for the list."""
+        self._copies.add(t.data_ptr())
+        return t
+
+    def _contiguous(self, t: torch.Tensor) -> torch.Tensor:
+        return t if t.is_contiguous() else self.adopt(t.contiguous())
 
     def _add(self, entry: str, args: tuple[int, ...], src: torch.Tensor, aux: Optional[torch.Tensor],
              dst: torch.Tensor, dst2: Optional[torch.Tensor] = None) -> None:
@@ -52,13 +68,18 @@ class Conversions:
         flat += (src.data_ptr(), aux.data_ptr() if aux is not None else 0, dst.data_ptr(),
                  dst2.data_ptr() if dst2 is not None else 0, n)  # struct FoConvRow
         keep.append((src, aux, dst, dst2))
-        self._held += src.numel() * src.element_size()
-        if self._held >= self.HELD:
+        self._work += src.nbytes
+        if self._copies:
+            for t in (src, aux):
+                if t is not None and t.data_ptr() in self._copies:
+                    self._copies.discard(t.data_ptr())
+                    self._held += t.nbytes
+        if self._held >= self.HELD or self._work >= self.WORK:
             self.launch()
 
     def launch(self) -> None:
         lists, self._lists = self._lists, {}
-        self._held = 0
+        self._held = self._work = 0
         for (entry, args, device), (flat, _) in lists.items():
             rows = array("q", flat)
             with torch.cuda.device(device):
@@ -70,8 +91,8 @@ class Conversions:
         """:func:`quantize` of a CUDA tensor."""
         x = x.detach()
         if x.dtype not in native.DTYPE_CODE:
-            x = x.to(torch.float32)
-        x = x.contiguous()
+            x = self.adopt(x.to(torch.float32))
+        x = self._contiguous(x)
         codes = torch.empty(x.shape, dtype=torch.int8 if signed else torch.uint8, device=x.device)
         scales = torch.empty(oracle.num_groups(x.numel()), dtype=torch.float16, device=x.device)
         self._add("fo_quantize_many", (native.DTYPE_CODE[x.dtype], int(signed), int(sqrt), int(softsign)),
@@ -83,7 +104,7 @@ class Conversions:
         """:func:`dequantize` of CUDA codes, rounded to bf16."""
         out = torch.empty(codes.shape, dtype=torch.bfloat16, device=codes.device)
         self._add("fo_dequantize_many", (native.FO_BF16, int(signed), int(sqrt), int(softsign)),
-                  codes.contiguous(), scales.contiguous(), out)
+                  self._contiguous(codes), self._contiguous(scales), out)
         return out
 
     def reconstruct_fp32_param(self, param: torch.Tensor, error_bits: torch.Tensor) -> torch.Tensor:
@@ -92,7 +113,7 @@ class Conversions:
             return reconstruct_fp32_param(param, error_bits)
         out = torch.empty(param.shape, dtype=torch.float32, device=param.device)
         self._add("fo_ecc_decode_many", (native.DTYPE_CODE[param.dtype], error_bits.element_size()),
-                  param.detach().contiguous(), error_bits.contiguous(), out)
+                  self._contiguous(param.detach()), self._contiguous(error_bits), out)
         return out
 
     def split(self, value: torch.Tensor, param: torch.Tensor, error_bits: torch.Tensor) -> Optional[torch.Tensor]:
@@ -103,7 +124,7 @@ class Conversions:
             return None
         codes = torch.empty(param.shape, dtype=error_bits.dtype, device=param.device)
         self._add("fo_ecc_split_many", (native.DTYPE_CODE[param.dtype], codes.element_size()),
-                  value.detach().contiguous(), None, param, codes)
+                  self._contiguous(value.detach()), None, param, codes)
         return codes
 
     def codes_as(self, codes: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:

@@ -656,7 +656,8 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
             # moments (either flavour) keep their checkpoint dtype until they are
             # re-quantised: a detour through an fp16 parameter dtype would flush
             # small second moments to zero, through bf16 it would round the scales
-            if isinstance(v, torch.Tensor) and (k in moment_keys or k.split("::")[0] in moment_keys):
+            if isinstance(v, torch.Tensor) and (k in moment_keys or k.split("::")[0] in moment_keys
+                                                or k == "error_bits"):
                 return _Shielded(v)
             return v
 
@@ -748,7 +749,13 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
                 p_local = local_tensor(param)
                 for key, val in list(pstate.items()):
                     if isinstance(val, _Shielded):
-                        pstate[key] = local_tensor(val.tensor).to(device=p_local.device)
+                        given = local_tensor(val.tensor)
+                        # correction codes travel as values of the parameter's dtype, and are cast to
+                        # it as torch would, but one by one
+                        moved = given.to(p_local.device)
+                        if key == "error_bits":
+                            moved = moved.to(p_local.dtype)
+                        pstate[key] = moved if moved is given else conversions.adopt(moved)
                     elif isinstance(val, torch.Tensor):
                         pstate[key] = local_tensor(val)
                 opt_state[param] = self._load_state_for_param(param, pstate, group, conversions)
@@ -804,7 +811,7 @@ class FlashOptimizer(torch.optim.Optimizer, abc.ABC):
             local_param = local_tensor(param.data)
             local_value = local_tensor(value)
             if local_value.device != local_param.device:
-                local_value = local_value.to(local_param.device)
+                local_value = conversions.adopt(local_value.to(local_param.device))
             state = self.state.get(param, {})
             if "error_bits" in state:
                 codes = conversions.split(local_value, local_param, state["error_bits"])

@@ -137,3 +137,62 @@ def test_import_from_host_memory_holds_few_copies_on_the_device(monkeypatch):
     torch.cuda.synchronize()
     assert torch.cuda.max_memory_allocated() - base < 24 * (4 << 20) + 96 * (1 << 20)  # new codes, and the copies in hand
     assert all((p == 1.0 + i).all() for i, p in enumerate(net))
+
+
+def _trained(count, numel):
+    net = nn.ParameterList([nn.Parameter(torch.full((numel,), 1.0, device="cuda").bfloat16()) for _ in range(count)])
+    opt = FlashAdamW(net.parameters(), lr=1e-3)
+    for p in net:
+        p.grad = torch.full_like(p, 1e-3)
+    opt.step()
+    opt.zero_grad()
+    return net, opt
+
+
+def _peak(fn):
+    torch.cuda.synchronize()
+    base = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    fn()
+    torch.cuda.synchronize()
+    return torch.cuda.max_memory_allocated() - base
+
+
+@pytest.mark.parametrize("what", ["checkpoint", "fp32 weights"])
+def test_host_memory_is_taken_in_with_few_copies_more_than_a_loop_holds(what, monkeypatch):
+    """192 MB of moments, or 384 MB of fp32 weights, in host memory: beyond what a loop over tensors
+    (a limit of nothing) holds, the limit and the tensors of the parameter in hand."""
+    net, opt = _trained(24, 1 << 22)
+    saved = opt.state_dict()
+    saved["state"] = {k: {n: v.cpu() for n, v in st.items()} for k, st in saved["state"].items()}
+    values = {k: torch.full((1 << 22,), 1.0 + i) for i, k in enumerate(net.state_dict())}
+
+    def run():
+        if what == "checkpoint":
+            opt.load_state_dict(saved)
+        else:
+            opt.set_fp32_model_state_dict(net, values)
+
+    run()
+    peak = _peak(run)
+    monkeypatch.setattr(Conversions, "HELD", 0)
+    assert peak - _peak(run) <= (32 << 20) + 3 * (16 << 20)
+
+
+def test_inputs_that_live_anyway_do_not_cut_a_list(monkeypatch):
+    monkeypatch.setattr(Conversions, "HELD", 1)
+    x = torch.randn(100, 64, device="cuda")
+    conv = Conversions()
+    codes, scales = conv.quantize(x, True, False, True)
+    conv.dequantize_bf16(codes, scales, True, False, True)
+    param = x.bfloat16()
+    error_bits = torch.empty(x.shape, dtype=torch.int8, device="cuda")
+    conv.split(x, param, error_bits)
+    conv.reconstruct_fp32_param(param, error_bits)
+    conv.codes_as(error_bits, torch.bfloat16)
+    assert len(conv._lists) == 5
+    codes, scales = conv.quantize(x.t(), True, False, True)  # of another layout: a copy, launched with the rest
+    assert not conv._lists
+    q_ref, s_ref = oracle.quantize_ref(x.t().cpu())
+    torch.cuda.synchronize()
+    assert torch.equal(codes.cpu(), q_ref) and torch.equal(scales.cpu(), s_ref)
