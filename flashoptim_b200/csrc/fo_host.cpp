@@ -297,6 +297,7 @@ Verdict visit(Walker* w, Group& g, const Call& c, PyObject* p) {
     const at::Tensor& sten = THPVariable_Unpack(so);
     if (!sten.is_cpu() || sten.scalar_type() != at::kFloat || sten.numel() != 1) return kFallback;
     float* counter = static_cast<float*>(sten.data_ptr());
+    if (!(*counter >= 0.0f && *counter < 1e9f)) return kFallback;
     step = (long long)(*counter + 1.0f);
     w->steps->push_back(counter);
   }
@@ -313,11 +314,11 @@ struct Hyper {
   int flag[3];
 };
 
-// 1 / (1 - beta^step); false when that is no number (the Python walk then raises).
+// 1 / (1 - beta^step); false outside the range where that is at least 1: the Python walk then
+// says what is wrong (a division by zero, a root of a negative number, an overflow).
 bool bias_correction(double beta, long long step, double& out) {
-  const double d = 1.0 - std::pow(beta, (double)step);
-  if (d == 0.0) return false;
-  out = 1.0 / d;
+  if (!(beta >= 0.0 && beta < 1.0) || step < 1) return false;
+  out = 1.0 / (1.0 - std::pow(beta, (double)step));
   return true;
 }
 

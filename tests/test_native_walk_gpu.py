@@ -229,3 +229,23 @@ def test_a_captured_step_keeps_its_address_table(native, monkeypatch):
         results.append(_state_tensors(opt))
     for (ka, a), (kb, b) in zip(*results):
         assert ka == kb and torch.equal(a, b), ka
+
+
+@pytest.mark.parametrize("native", [True, False])
+@pytest.mark.parametrize("betas,count,error", [
+    ((0.9, 1.5), 1.0, ValueError), ((1.5, 0.9), 1e6, OverflowError), ((0.9, 1.0), 1.0, ZeroDivisionError),
+    ((0.9, 0.999), -3.0, ValueError), ((0.9, 0.999), float("nan"), ValueError),
+])
+def test_moment_factors_and_step_counts_without_a_bias_correction_are_refused(native, betas, count, error, monkeypatch):
+    p = nn.Parameter(torch.ones(100, device="cuda").bfloat16())
+    opt = fo.FlashAdamW([p], lr=0.1)
+    if not native:
+        monkeypatch.setattr(opt, "_native_step_group", lambda *a: False)
+    p.grad = torch.ones_like(p)
+    opt.step()
+    before = p.detach().clone()
+    opt.param_groups[0]["betas"] = betas
+    opt.state[p]["step"].fill_(count)
+    with pytest.raises(error):
+        opt.step()
+    assert torch.equal(p, before)
