@@ -120,10 +120,15 @@ struct Group {
   long long calls = 0;
 };
 
+struct Counter {
+  float* at;
+  float was;
+};
+
 struct Walker {
   PyObject_HEAD
   std::vector<Group>* groups;
-  std::vector<float*>* steps;       // Adam step counters to advance
+  std::vector<Counter>* steps;      // Adam step counters to advance
   std::vector<PyObject*>* updated;  // parameters of this call that the launches update (borrowed)
   std::vector<PyObject*>* skipped;  // those that a collective-fused update has done already (borrowed)
   bool busy;
@@ -299,7 +304,7 @@ Verdict visit(Walker* w, Group& g, const Call& c, PyObject* p) {
     float* counter = static_cast<float*>(sten.data_ptr());
     if (!(*counter >= 0.0f && *counter < 1e9f)) return kFallback;
     step = (long long)(*counter + 1.0f);
-    w->steps->push_back(counter);
+    w->steps->push_back({counter, *counter});
   }
   Bucket& b = bucket_for(g, t.device().index(), dtype, err, mode, step);
   b.rows.push_back(row);
@@ -539,6 +544,14 @@ PyObject* walker_step(Walker* w, PyObject* const* args, Py_ssize_t nargs) {
       upload(g, b);
     }
 
+    // a counter that several parameters share advances once for each before any of them is read
+    bool shared = false;
+    for (const Counter& s : *w->steps) *s.at += 1.0f;
+    for (const Counter& s : *w->steps) shared = shared || *s.at != s.was + 1.0f;
+    if (shared) {
+      for (const Counter& s : *w->steps) *s.at = s.was;
+      Py_RETURN_FALSE;
+    }
     // from here on the call is committed
     for (PyObject* p : *w->skipped) {
       PyObject* id = PyLong_FromVoidPtr(p);
@@ -548,7 +561,6 @@ PyObject* walker_step(Walker* w, PyObject* const* args, Py_ssize_t nargs) {
       }
       Py_DECREF(id);
     }
-    for (float* s : *w->steps) *s += 1.0f;
     for (size_t i = 0; i < g.used; ++i) {
       static const FoAdamHyper none = {};
       int rc;
@@ -577,7 +589,7 @@ PyObject* walker_new(PyTypeObject* type, PyObject*, PyObject*) {
   Walker* w = reinterpret_cast<Walker*>(type->tp_alloc(type, 0));
   if (!w) return nullptr;
   w->groups = new std::vector<Group>();
-  w->steps = new std::vector<float*>();
+  w->steps = new std::vector<Counter>();
   w->updated = new std::vector<PyObject*>();
   w->skipped = new std::vector<PyObject*>();
   w->busy = false;

@@ -249,3 +249,20 @@ def test_moment_factors_and_step_counts_without_a_bias_correction_are_refused(na
     with pytest.raises(error):
         opt.step()
     assert torch.equal(p, before)
+
+
+def test_a_step_count_that_parameters_share(monkeypatch):
+    results = []
+    for native in (True, False):
+        params = [nn.Parameter(torch.linspace(-1, 1, 700 + i, device="cuda").bfloat16()) for i in range(5)]
+        opt = fo.FlashAdamW(params, lr=0.01)
+        if not native:
+            monkeypatch.setattr(opt, "_native_step_group", lambda *a: False)
+        for it in range(3):
+            _grads(params, it, ())
+            opt.step()
+            for p in params[1:3]:
+                opt.state[p]["step"] = opt.state[params[0]]["step"]
+        results.append(_state_tensors(opt))
+    for (ka, a), (kb, b) in zip(*results):
+        assert ka == kb and torch.equal(a, b), ka
