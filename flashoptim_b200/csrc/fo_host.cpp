@@ -14,6 +14,7 @@
 // (flashoptim/optimizers.py:1535-1583, :2203-2252).
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/utils/object_ptr.h>
 
 #include <ATen/ATen.h>
 #include <ATen/core/grad_mode.h>
@@ -131,6 +132,9 @@ struct Walker {
   std::vector<Counter>* steps;      // Adam step counters to advance
   std::vector<PyObject*>* updated;  // parameters of this call that the launches update (borrowed)
   std::vector<PyObject*>* skipped;  // those that a collective-fused update has done already (borrowed)
+  // kept until the call is launched, whatever Python code runs meanwhile lets go of
+  std::vector<at::Tensor>* held;        // parameters and gradients
+  std::vector<PyObject*>* held_states;  // and the dictionaries of their states
   bool busy;
 };
 
@@ -309,6 +313,9 @@ Verdict visit(Walker* w, Group& g, const Call& c, PyObject* p) {
   Bucket& b = bucket_for(g, t.device().index(), dtype, err, mode, step);
   b.rows.push_back(row);
   w->updated->push_back(p);
+  w->held->push_back(std::move(t));
+  w->held->push_back(std::move(grad));
+  w->held_states->push_back(Py_NewRef(st));
   return kOk;
 }
 
@@ -457,10 +464,16 @@ struct GilReleased {
   ~GilReleased() { PyEval_RestoreThread(state); }
 };
 
+// One call of a walker.  What it holds is let go under the GIL, which its owner has at the end.
 struct Busy {
-  bool& b;
-  explicit Busy(bool& f) : b(f) { b = true; }
-  ~Busy() { b = false; }
+  Walker* w;
+  explicit Busy(Walker* walker) : w(walker) { w->busy = true; }
+  ~Busy() {
+    w->held->clear();
+    for (PyObject* st : *w->held_states) Py_DECREF(st);
+    w->held_states->clear();
+    w->busy = false;
+  }
 };
 
 // Nothing is done for an optimizer with methods of its own in the walk's place.
@@ -508,9 +521,12 @@ PyObject* walker_step(Walker* w, PyObject* const* args, Py_ssize_t nargs) {
     h.v[i] = PyFloat_AsDouble(v);
     if (h.v[i] == -1.0 && PyErr_Occurred()) return nullptr;
   }
-  for (Py_ssize_t i = 0; i < n_flags; ++i) h.flag[i] = PyObject_IsTrue(PyTuple_GET_ITEM(args[11], n_vals + i));
+  for (Py_ssize_t i = 0; i < n_flags; ++i) {
+    h.flag[i] = PyObject_IsTrue(PyTuple_GET_ITEM(args[11], n_vals + i));
+    if (h.flag[i] < 0) return nullptr;
+  }
 
-  Busy busy(w->busy);
+  Busy busy(w);
   at::NoGradGuard no_grad;  // for the Python methods that the walk calls: state creation, numerics check
   try {
     // groups are numbered from -1 (a group dict that the optimizer does not own)
@@ -534,6 +550,11 @@ PyObject* walker_step(Walker* w, PyObject* const* args, Py_ssize_t nargs) {
       if (c.adam && !adam_hyper(h, g.buckets[i]->step, ah[i])) Py_RETURN_FALSE;
     }
     if (!c.adam) momentum_hyper(h, mh);
+    // taken down before the GIL is given away, after which the group's list is no longer ours
+    THPObjectPtr list(c.listeners ? PyList_New((Py_ssize_t)w->updated->size()) : nullptr);
+    if (c.listeners && !list) return nullptr;
+    for (size_t i = 0; c.listeners && i < w->updated->size(); ++i)
+      PyList_SET_ITEM(list.get(), (Py_ssize_t)i, Py_NewRef((*w->updated)[i]));
     for (size_t i = 0; i < g.used; ++i)
       if (!ensure_status(g.buckets[i]->device)) return nullptr;
     for (size_t i = 0; i < g.used; ++i) {
@@ -575,10 +596,7 @@ PyObject* walker_step(Walker* w, PyObject* const* args, Py_ssize_t nargs) {
       ++g_launches;
     }
     if (!c.listeners) Py_RETURN_TRUE;
-    PyObject* list = PyList_New((Py_ssize_t)w->updated->size());
-    if (!list) return nullptr;
-    for (size_t i = 0; i < w->updated->size(); ++i) PyList_SET_ITEM(list, i, Py_NewRef((*w->updated)[i]));
-    return list;
+    return list.release();
   } catch (...) {  // as the Python exception that torch makes of it, OutOfMemoryError among them
     if (!PyErr_Occurred()) torch::translate_exception_to_python(std::current_exception());
     return nullptr;
@@ -592,6 +610,8 @@ PyObject* walker_new(PyTypeObject* type, PyObject*, PyObject*) {
   w->steps = new std::vector<Counter>();
   w->updated = new std::vector<PyObject*>();
   w->skipped = new std::vector<PyObject*>();
+  w->held = new std::vector<at::Tensor>();
+  w->held_states = new std::vector<PyObject*>();
   w->busy = false;
   return reinterpret_cast<PyObject*>(w);
 }
@@ -614,6 +634,8 @@ void walker_dealloc(Walker* w) {
   delete w->steps;
   delete w->updated;
   delete w->skipped;
+  delete w->held;
+  delete w->held_states;
   Py_TYPE(w)->tp_free(reinterpret_cast<PyObject*>(w));
 }
 

@@ -266,3 +266,34 @@ def test_a_step_count_that_parameters_share(monkeypatch):
         results.append(_state_tensors(opt))
     for (ka, a), (kb, b) in zip(*results):
         assert ka == kb and torch.equal(a, b), ka
+
+
+@pytest.mark.parametrize("lost", ["gradient", "state"])
+def test_what_goes_during_the_walk_is_kept_until_the_launch(lost, monkeypatch):
+    """A method that the walk calls drops a gradient, or replaces a state, that was looked at before,
+    and its memory is used again at once."""
+    results = []
+    for native in (True, False):
+        class Lion(fo.FlashLion):
+            def _check_param_numerics(self, p, *args):
+                if p is params[2] and armed:
+                    if lost == "gradient":
+                        params[0].grad = None
+                    else:
+                        self.state[params[0]] = {}
+                    armed.append([torch.full((1 << 20,), float("nan"), device="cuda") for _ in range(8)])
+
+        params = [nn.Parameter(torch.linspace(-1, 1, 1 << 21, device="cuda").bfloat16()) for _ in range(4)]
+        opt = Lion(params, lr=0.01, check_numerics=True)
+        if not native:
+            monkeypatch.setattr(opt, "_native_step_group", lambda *a: False)
+        armed = []
+        for p in params:
+            p.grad = torch.linspace(-1, 1, 1 << 21, device="cuda").bfloat16()
+        opt.step()
+        armed.append(True)
+        opt.step()
+        torch.cuda.synchronize()
+        results.append([p.detach().cpu() for p in params])
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
