@@ -9,8 +9,8 @@
 // use, so states may be replaced, emptied or loaded at any time.
 //
 // A group that this walk does not serve (CPU or non-contiguous tensors, a gradient of another
-// dtype, ...) is left untouched and reported to the caller, whose Python walk updates it or says
-// what is wrong with it.  It takes the place of the per-tensor launch wrappers of the reference
+// dtype, an optimizer with methods of its own in the walk's place, ...) is left untouched and
+// reported to the caller, whose Python walk updates it or says what is wrong with it.  It takes the place of the per-tensor launch wrappers of the reference
 // (flashoptim/optimizers.py:1535-1583, :2203-2252).
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>

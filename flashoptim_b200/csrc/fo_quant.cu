@@ -1,10 +1,11 @@
 // Stand-alone group quantiser / dequantiser, master-weight split and maxabs.
 //
-// These run at checkpoint save/load, fp32 export/import and when a state is set
-// from a full-precision tensor (never inside a training step), so
-// they use exact IEEE arithmetic (explicit round-to-nearest intrinsics, which
-// the compiler never contracts into FMAs) and reproduce the PyTorch formulation
-// in ops/oracle.py bit for bit.  What they compute matches
+// These run at checkpoint save/load, fp32 export/import and when a state is set from a
+// full-precision tensor, never inside a training step, and reproduce the PyTorch formulation in
+// ops/oracle.py bit for bit.  The quantiser takes an approximate reciprocal where its error cannot
+// change the code and the formula's IEEE operations elsewhere; the dequantiser's quotients are
+// corrected by their exact remainders; the master-weight kernels use round-to-nearest intrinsics,
+// which the compiler never contracts into FMAs.  What they compute matches
 // flashoptim/optimizers.py:2610-2676 (quantise), :2541-2607 (dequantise),
 // :2726-2776 (error-correction encode / decode).
 #include <type_traits>
@@ -699,15 +700,11 @@ __global__ void __launch_bounds__(kQThreads) maxabs_kernel(const T* __restrict__
   if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<unsigned int*>(out), __float_as_uint(a));
 }
 
-// Grid: a grid-stride loop over at most 128 CTAs per SM (the SM count is read once per device),
-// never more than the work.  Measured on B200 with 2^28 elements: a grid of exactly the
-// resident CTAs (one round, equal shares) was 10 % slower for the quantiser, because the SMs do
-// not all run at the same pace and a fixed share per CTA waits for the slowest; 16 per SM lost
-// to round quantisation (2.7-3.2 rounds at a residency of 5-6); 24 / 32 / 48 / 128 per SM got
-// faster in that order; one unit per thread over the whole grid (no loop) was slower again for
-// five of the seven kernels.  -DFO_QUANT_BLOCKS_PER_SM=k changes the factor for tuning builds.
-// The kernels over lists, whose chunk is twice as large, cap their grids accordingly (quantiser at
-// 2^28 elements: 168 us with 16 CTAs per SM, 158 with 64, 166 with 256).
+// Grids: a loop over chunks by at most 64 CTAs per SM (the SM count is read once per device), never
+// more than the work.  Several times the resident CTAs, because the SMs do not all run at the same
+// pace and equal fixed shares wait for the slowest (quantiser at 2^28 elements: 168 us with 16 CTAs
+// per SM, 158 with 64, 166 with 256).  maxabs, whose units are half as large, takes twice as many;
+// -DFO_QUANT_BLOCKS_PER_SM=k changes that for tuning builds.
 constexpr int kListCtasPerSm = 64;
 #ifndef FO_QUANT_BLOCKS_PER_SM
 #define FO_QUANT_BLOCKS_PER_SM 128

@@ -7,14 +7,15 @@
 // streams whole chunks (parameter, gradient, correction codes, state codes and
 // their scales: 14-21 KB) into a ring of shared-memory stages with
 // cp.async.bulk (the TMA unit's untiled copy; no multicast, no tensor map),
-// completion is tracked by one mbarrier per stage, and eight consumer warps read
-// their units from shared memory, release the stage and run the same update
-// and stores as the register path.  Up to kStages - 1 chunks per CTA are in
+// completion is tracked by one mbarrier per stage, and four consumer warps read
+// 16 elements per thread from shared memory, release the stage and run the same
+// update as the register path.  Up to kStages - 1 chunks per CTA are in
 // flight regardless of what the consumers are doing.
 //
-// A chunk that is not a full, 16-byte aligned 2048-element block (tails,
-// tensors at odd offsets) skips the copy engine: the producer completes the
-// stage's phase with a plain arrive and the consumers load it directly.
+// A chunk that is not a full 2048-element block (a tail), or whose parameter or
+// states do not start on 16 bytes, skips the copy engine: the producer completes
+// the stage's phase with a plain arrive and the consumers load it directly.  The
+// gradient may start anywhere (chunk_is_staged).
 //
 // Every mbarrier wait is bounded (wall clock); a wait that runs out records a
 // code in StepParams.status (when given), and the waiting warp leaves its loop.
@@ -26,8 +27,8 @@ namespace fo {
 // A consumer thread owns kSpan = 16 consecutive elements of a chunk, half a quantisation group:
 // the group's absmax takes one shuffle, codes move as 16-byte vectors, and what a thread spends per
 // chunk outside the arithmetic (barrier, addresses, constants, scales) is shared by 16 elements.
-// These kernels are bound by instruction issue and, through it, by the power cap (the clock falls
-// to 1.63 of 1.965 GHz within 0.1 s).
+// These kernels are bound by instruction issue (43 per AdamW element, 67 % of the issue slots) and,
+// through it, by the power cap: 1.53-1.56 of 1.965 GHz at 998 W over 150 steps of 8.03 B elements.
 constexpr int kSpan = 16;
 constexpr int kStagedChunk = kChunk;  // elements; the chunk prefix is shared with the register path
 constexpr int kConsumerThreads = kStagedChunk / kSpan;

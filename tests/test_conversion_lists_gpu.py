@@ -120,9 +120,8 @@ def test_what_the_list_kernels_do_not_serve_is_converted_all_the_same():
     assert (net.a == 1).all() and (opt.state[net.a]["error_bits"] == 0).all()
 
 
-def test_import_from_host_memory_holds_few_copies_on_the_device(monkeypatch):
+def test_import_from_host_memory_holds_few_copies_on_the_device():
     """24 fp32 tensors of 16 MB: 384 MB if every device copy waited for one launch at the end."""
-    monkeypatch.setattr(Conversions, "HELD", 32 << 20)
     net = nn.ParameterList([nn.Parameter(torch.zeros(1 << 22, device="cuda", dtype=torch.bfloat16)) for _ in range(24)])
     opt = FlashAdamW(net.parameters(), lr=1e-3)
     for p in net:

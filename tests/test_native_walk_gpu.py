@@ -297,3 +297,38 @@ def test_what_goes_during_the_walk_is_kept_until_the_launch(lost, monkeypatch):
         results.append([p.detach().cpu() for p in params])
     for a, b in zip(*results):
         assert torch.equal(a, b)
+
+
+def test_sharded_parameters_are_walked_as_in_python(monkeypatch):
+    """DTensors (parameters and gradients) on a mesh of one, with more rows than fit the parameters."""
+    import torch.distributed as dist
+    from torch.distributed.device_mesh import init_device_mesh
+    from torch.distributed.tensor import DTensor, Replicate, Shard
+
+    dist.init_process_group("nccl", store=dist.HashStore(), rank=0, world_size=1)
+    try:
+        mesh = init_device_mesh("cuda", (1,))
+        results = []
+        for native in (True, False):
+            g = torch.Generator().manual_seed(5)
+
+            def sharded(i, dtype):
+                t = torch.randn((33, 1025, 4096, 7)[i % 4] + i, generator=g).to(dtype).cuda()
+                return DTensor.from_local(t, mesh, [Shard(0) if i % 3 else Replicate()])
+
+            dtypes = [torch.float32 if i % 5 == 4 else torch.bfloat16 for i in range(24)]
+            params = [nn.Parameter(sharded(i, d)) for i, d in enumerate(dtypes)]
+            opt = fo.FlashAdamW(params, lr=0.01)
+            if not native:
+                monkeypatch.setattr(opt, "_native_step_group", lambda *a: False)
+            for _ in range(3):
+                for i, (p, d) in enumerate(zip(params, dtypes)):
+                    p.grad = sharded(i, d)
+                opt.step()
+            assert native == bool(opt._walker is not None and opt._walker.tables())
+            torch.cuda.synchronize()
+            results.append([(k, t.to_local() if isinstance(t, DTensor) else t) for k, t in _state_tensors(opt)])
+        for (ka, a), (kb, b) in zip(*results):
+            assert ka == kb and torch.equal(a, b), ka
+    finally:
+        dist.destroy_process_group()

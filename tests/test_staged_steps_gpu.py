@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 
 # long enough together for the staged kernels to be chosen; tails of every kind behind them
 SIZES = (1, 2047, 2048, 2049, 31, 1_500_017, 4096, 65_537, 33, 500_000)
-MANY = (1024,) * 700 + (2048,) * 40 + (5,) * 30 + (1_000_003,)  # segment look-up over many tensors
+MANY = (1024,) * 700 + (2048,) * 40 + (5,) * 30 + (1_300_003,)  # segment look-up over many tensors
 
 
 def _streams(sizes, dtype, err, n_states, skew, seed):
@@ -81,6 +81,9 @@ def test_staged_equals_register_path(dtype, err, n_states, skew):
 @pytest.mark.parametrize("count", [len(MANY), 17, 33, 64])
 def test_segment_look_up_over_many_tensors(count):
     sizes = MANY[-count:]
+    # more chunks than the register path has CTAs: the staged kernel is the one that runs
+    chunk = native.chunk_elems()
+    assert sum(-(-n // chunk) for n in sizes) > native.load().fo_step_grid(torch.cuda.current_device())
     results = []
     for variant in (0, 1):
         rows, bufs, _ = _streams(sizes, torch.bfloat16, 1, 2, 0, seed=3)
