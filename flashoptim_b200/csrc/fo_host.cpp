@@ -71,23 +71,39 @@ PyObject* slot(PyObject* o, Py_ssize_t off) {  // borrowed; null for None or nev
 // keeps those that it describes in `_walked_natively` (optim/base.py).
 PyObject* g_walked = nullptr;
 
+// A class as it was looked at last: the interpreter gives a class another version whenever it, or a
+// class above it, is changed.
+struct Looked {
+  PyTypeObject* type = nullptr;
+  unsigned int version = 0;
+};
+
 // Whether the class of `opt`, or `opt` itself, has other methods than those; -1 with an exception.
-int overrides(PyObject* opt) {
-  PyObject* type = reinterpret_cast<PyObject*>(Py_TYPE(opt));
-  PyObject* known = PyObject_GetAttr(type, s_walked_natively);
-  if (!known) return -1;
-  PyObject* own = PyObject_GenericGetDict(opt, nullptr);
+// Every call asks, so a class that is as it was is not looked through again.
+int overrides(PyObject* opt, Looked& last) {
+  PyTypeObject* type = Py_TYPE(opt);
   const Py_ssize_t n = PyTuple_GET_SIZE(g_walked);
-  int other = own ? !PyTuple_Check(known) || PyTuple_GET_SIZE(known) != n : -1;
-  for (Py_ssize_t i = 0; !other && i < n; ++i) {
-    PyObject* name = PyTuple_GET_ITEM(g_walked, i);
-    PyObject* now = PyObject_GetAttr(type, name);
-    other = now ? now != PyTuple_GET_ITEM(known, i) : -1;
-    Py_XDECREF(now);
-    if (!other) other = PyDict_Contains(own, name);
+  if (last.type != type || !PyType_HasFeature(type, Py_TPFLAGS_VALID_VERSION_TAG) || type->tp_version_tag == 0 ||
+      type->tp_version_tag != last.version) {
+    last.type = nullptr;
+    PyObject* cls = reinterpret_cast<PyObject*>(type);
+    PyObject* known = PyObject_GetAttr(cls, s_walked_natively);
+    if (!known) return -1;
+    int other = !PyTuple_Check(known) || PyTuple_GET_SIZE(known) != n;
+    for (Py_ssize_t i = 0; !other && i < n; ++i) {
+      PyObject* now = PyObject_GetAttr(cls, PyTuple_GET_ITEM(g_walked, i));
+      other = now ? now != PyTuple_GET_ITEM(known, i) : -1;
+      Py_XDECREF(now);
+    }
+    Py_DECREF(known);
+    if (other) return other;
+    last.type = type;
+    last.version = type->tp_version_tag;
   }
+  PyObject* own = PyObject_GenericGetDict(opt, nullptr);
+  int other = own ? 0 : -1;
+  for (Py_ssize_t i = 0; !other && i < n; ++i) other = PyDict_Contains(own, PyTuple_GET_ITEM(g_walked, i));
   Py_XDECREF(own);
-  Py_DECREF(known);
   return other;
 }
 
@@ -135,6 +151,7 @@ struct Walker {
   // kept until the call is launched, whatever Python code runs meanwhile lets go of
   std::vector<at::Tensor>* held;        // parameters and gradients
   std::vector<PyObject*>* held_states;  // and the dictionaries of their states
+  Looked* looked;
   bool busy;
 };
 
@@ -207,6 +224,7 @@ Verdict visit(Walker* w, Group& g, const Call& c, PyObject* p) {
   Py_DECREF(id);
   if (ready < 0 || skip < 0) return kError;
   if (!st || !ready || !PyDict_Check(st) || PyDict_GET_SIZE(st) == 0 || c.check) {
+    at::NoGradGuard no_grad;
     PyObject* r = PyObject_CallMethodObjArgs(c.opt, s_ensure, p, c.group, nullptr);
     if (!r) return kError;
     Py_DECREF(r);
@@ -240,6 +258,7 @@ Verdict visit(Walker* w, Group& g, const Call& c, PyObject* p) {
       !grad.is_contiguous() || grad.scalar_type() != t.scalar_type() || grad.numel() != n)
     return kFallback;
   if (c.check) {
+    at::NoGradGuard no_grad;
     PyObject* r = PyObject_CallMethodObjArgs(c.opt, s_check, p, c.lr, c.width, nullptr);
     if (!r) return kError;
     Py_DECREF(r);
@@ -485,7 +504,7 @@ PyObject* walker_step(Walker* w, PyObject* const* args, Py_ssize_t nargs) {
     return nullptr;
   }
   if (w->busy) Py_RETURN_FALSE;  // another thread is inside a launch of this optimizer
-  if (const int other = overrides(args[0])) {
+  if (const int other = overrides(args[0], *w->looked)) {
     if (other < 0) return nullptr;
     Py_RETURN_FALSE;
   }
@@ -527,7 +546,6 @@ PyObject* walker_step(Walker* w, PyObject* const* args, Py_ssize_t nargs) {
   }
 
   Busy busy(w);
-  at::NoGradGuard no_grad;  // for the Python methods that the walk calls: state creation, numerics check
   try {
     // groups are numbered from -1 (a group dict that the optimizer does not own)
     const size_t slot_index = (size_t)(c.group_index + 1);
@@ -612,6 +630,7 @@ PyObject* walker_new(PyTypeObject* type, PyObject*, PyObject*) {
   w->skipped = new std::vector<PyObject*>();
   w->held = new std::vector<at::Tensor>();
   w->held_states = new std::vector<PyObject*>();
+  w->looked = new Looked();
   w->busy = false;
   return reinterpret_cast<PyObject*>(w);
 }
@@ -636,6 +655,7 @@ void walker_dealloc(Walker* w) {
   delete w->skipped;
   delete w->held;
   delete w->held_states;
+  delete w->looked;
   Py_TYPE(w)->tp_free(reinterpret_cast<PyObject*>(w));
 }
 
@@ -686,7 +706,8 @@ PyObject* host_setup(PyObject*, PyObject* args) {
 PyObject* host_launches(PyObject*, PyObject*) { return PyLong_FromLongLong(g_launches); }
 
 PyObject* host_overrides(PyObject*, PyObject* opt) {
-  const int other = overrides(opt);
+  Looked nothing_yet;
+  const int other = overrides(opt, nothing_yet);
   return other < 0 ? nullptr : PyBool_FromLong(other);
 }
 

@@ -42,6 +42,33 @@ def test_an_override_keeps_the_native_walk_out(cls, name, monkeypatch):
     assert host.load().overrides(opt)
 
 
+@pytest.mark.gpu
+def test_a_class_or_an_optimizer_that_changes_between_steps(monkeypatch):
+    """The look at a class is remembered until the class, or one above it, changes."""
+    class Lion(fo.FlashLion):
+        pass
+
+    calls = []
+    p = _param("cuda")
+    opt = Lion([p], lr=0.1)
+
+    def steps():
+        calls.clear()
+        for _ in range(2):
+            p.grad = torch.ones_like(p)
+            opt.step()
+        return len(calls)
+
+    original = fo.FlashLion._pre_step
+    patched = lambda self, state: calls.append(original(self, state))  # noqa: E731
+    assert steps() == 0
+    for owner in (Lion, fo.FlashLion, opt):
+        with monkeypatch.context() as m:
+            m.setattr(owner, "_pre_step", patched if owner is not opt else lambda state: calls.append(state))
+            assert steps() == 2
+        assert steps() == 0
+
+
 def test_a_class_that_says_what_it_does_is_walked_natively():
     class Own(fo.FlashLion):
         def _pre_step_many(self, param_states):
